@@ -7,7 +7,7 @@
 //   by HBM footprint against a byte budget.
 // * A step is two persistent launches per Riemann solver in use (Heun stages; HLLD solves and
 //   HLLC solves in separate launches, so each kernel holds one solver body) whose CTAs draw
-//   32x7xlz tiles of those solves from one work-queue counter; each solve counts its own tiles,
+//   column tiles of those solves from one work-queue counter; each solve counts its own tiles,
 //   so each keeps its own lagged dt and clock.  While membership is unchanged the launch sequence of a chunk of steps
 //   is replayed from a captured CUDA graph.
 // * The z-march length lz and the persistent grid size are chosen by an autotuner that times
@@ -260,7 +260,7 @@ int launch_items(setb_batch* b, int stage, int n_state, unsigned* q) {
     const int n = n_state == 3 ? b->n_hlld : b->n_items - b->n_hlld;
     if (n == 0) return SETB_OK;
     BatchArgs a{stage == 1 ? b->d_inst1 : b->d_inst2, b->d_items + first, n, q};
-    SB_TRY(launch_batch_stage(a, b->precision, n_state, stage == 1 ? 0 : 1, stage == 1, grid_size(b, n), b->stream));
+    SB_TRY(launch_batch_stage(a, b->precision, n_state, stage == 1 ? 0 : 1, grid_size(b, n), b->stream));
     return SETB_OK;
 }
 

@@ -647,7 +647,7 @@ int enqueue_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaE
             a.Uout = W;
             a.finalize = 0;
             a.comp = nullptr;
-            SB_TRY(launch_stage(a, P, o->n_state, o->order, 0, true, h->stream));
+            SB_TRY(launch_stage(a, P, o->n_state, o->order, 0, h->stream));
             if (ev) SB_TRY(cudaEventRecord(ev[2 * s + 1], h->stream));
             a.g.lz = lz1;
             a.Uin = W;
@@ -656,7 +656,7 @@ int enqueue_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaE
             a.Uout = U;
             a.finalize = 1;
             a.comp = comp;
-            SB_TRY(launch_stage(a, P, o->n_state, o->order, 1, false, h->stream));
+            SB_TRY(launch_stage(a, P, o->n_state, o->order, 1, h->stream));
             if (ev) SB_TRY(cudaEventRecord(ev[2 * s + 2], h->stream));
         } else {
             a.g.lz = lz0;
@@ -666,7 +666,7 @@ int enqueue_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaE
             a.Uout = W;
             a.finalize = 1;
             a.comp = comp;
-            SB_TRY(launch_stage(a, P, o->n_state, o->order, 0, true, h->stream));
+            SB_TRY(launch_stage(a, P, o->n_state, o->order, 0, h->stream));
             if (ev) {
                 SB_TRY(cudaEventRecord(ev[2 * s + 1], h->stream));
                 SB_TRY(cudaEventRecord(ev[2 * s + 2], h->stream));
@@ -922,7 +922,7 @@ int32_t setb_slab_stage(setb_handle* h, int32_t stage, const setb_step_opts* o) 
         a.finalize = 1;
         a.comp = comp;
     }
-    SB_TRY(launch_stage(a, P, o->n_state, o->order, kind, stage == 1, h->stream));
+    SB_TRY(launch_stage(a, P, o->n_state, o->order, kind, h->stream));
     if (stage == 1 && o->scheme == 1) h->cur = 1 - h->cur;
     return SETB_OK;
 }

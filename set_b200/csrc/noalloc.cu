@@ -139,19 +139,19 @@ extern "C" int32_t setb_step_noalloc(const setb_cart_desc* d, const setb_step_op
             a.Ubase = nullptr;
             a.Uout = other;
             a.finalize = 0;
-            e = launch_stage_fp64(a, o->n_state, o->order, 0, true, s);
+            e = launch_stage(a, 0, o->n_state, o->order, 0, s);
             if (e != cudaSuccess) return SETB_ECUDA;
             a.Uin = other;
             a.Ubase = cur;
             a.Uout = cur;
             a.finalize = 1;
-            e = launch_stage_fp64(a, o->n_state, o->order, 1, false, s);
+            e = launch_stage(a, 0, o->n_state, o->order, 1, s);
         } else {
             a.Uin = cur;
             a.Ubase = nullptr;
             a.Uout = other;
             a.finalize = 1;
-            e = launch_stage_fp64(a, o->n_state, o->order, 0, true, s);
+            e = launch_stage(a, 0, o->n_state, o->order, 0, s);
             double* t = cur;
             cur = other;
             other = t;

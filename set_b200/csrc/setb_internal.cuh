@@ -8,30 +8,29 @@
 
 namespace sb {
 
+// Column tile of the stage kernels: kTileX x ty cells marched along z by `threads` threads, one warp
+// per tile row and one for the tile's edges, `ctas_per_sm` resident per SM, `boxes` staged planes.
+// The plain and delta forms' FP64 ring limits the tile to 11 rows (223 KB of shared memory; 12
+// warps of 168 registers: 16 warps of 128 with 10 rows spill, 2.65 / 2.74 against 2.31 / 2.44 ms a
+// stage at 256^3 when it was tried).  The mixed form's FP32 ring leaves room for 15 rows: 16 warps
+// of 128 registers and the smallest halo (1.43 cells staged per cell; 384^3, stage 1 / 2: 4.82 /
+// 5.58 ms against 5.32 / 6.12 with 11 rows and 12 warps).  Its two staged boxes would fit, but leave
+// 18 KB of L1 for the second stage's loads: 6.32 against 5.58 ms.
+constexpr int kTileX = 32;
+struct TileShape {
+    int ty, threads, ctas_per_sm, boxes;
+};
+SB_HD constexpr TileShape tile_shape(int precision, int kind) {
+    (void)kind;
+    return precision == 1 ? TileShape{15, 512, 1, 1} : TileShape{11, 384, 1, 1};
+}
+// The tile_shape kind every batch launch uses.
+constexpr int kBatchKind = 1;
+
 // Clock of one solve, in device memory.  The reference keeps time_step / time_step2 /
 // dev_time_all as device scalars written from the host each step (cuf_kernel.cuf:18-19,
 // 789-794); here the last CTA of each step's final kernel rolls the clock on the device, so a
 // run of steps needs no host round trip.
-// Column tile of the stage kernels: kTileX x ty cells marched along z by `threads` threads,
-// `ctas_per_sm` resident per SM; per form (precision 0 plain FP64, 1 mixed, 2 delta) and launch
-// (kind 0: Euler step / Heun stage 1; kind 1: Heun stage 2 and every batch launch).  The plain
-// and delta forms fit FP64 HLLD in 168 registers (384 threads, 12 warps per SM).  The mixed
-// form's first stage runs that shape too; its second stage, which also streams the FP32
-// compensation, runs two 256-thread CTAs of at most 128 registers, so one CTA's update overlaps
-// the other's faces.
-constexpr int kTileX = 32;
-struct TileShape {
-    int ty, threads, ctas_per_sm;
-};
-SB_HD constexpr TileShape tile_shape(int precision, int kind) {
-    return (precision == 1 && kind == 1) ? TileShape{7, 256, 2} : TileShape{11, 384, 1};
-}
-// The tile_shape kind every batch launch uses.  The batch kernel holds the HLLC and HLLD bodies;
-// in the mixed form the kind-1 shape (two 256-thread CTAs per SM, 128 registers, ~320 B of
-// spills) measured 1.5 % faster on the 64-grid ensemble than the kind-0 shape (one 384-thread
-// CTA, 168 registers, ~80 B of spills).
-constexpr int kBatchKind = 1;
-
 struct DevClock {
     double dt_cur;                  // dt used by the current step (time_step)
     unsigned long long dt_next;     // bits of the running min for the next step (time_step2)
@@ -381,13 +380,13 @@ cudaError_t fl_launch_stage(const FaceListDev* f, const double* Uin, const doubl
                             bool finalize, cudaStream_t s);
 
 // ---------------------------------------------------------------- launch entry points
-cudaError_t launch_stage_fp64(const StageArgs& a, int n_state, int order, int kind, bool want_dt,
-                              cudaStream_t s);
-cudaError_t launch_stage(const StageArgs& a, int precision, int n_state, int order, int kind, bool want_dt,
-                         cudaStream_t s);
-int stage_smem_bytes(int precision, int kind);
-cudaError_t launch_batch_stage(const BatchArgs& b, int precision, int n_state, int kind, bool want_dt, int grid,
-                               cudaStream_t s);
+// kind 0: Euler step / Heun stage 1 (reduces the dt candidate), kind 1: Heun stage 2.
+cudaError_t launch_stage(const StageArgs& a, int precision, int n_state, int order, int kind, cudaStream_t s);
+cudaError_t launch_batch_stage(const BatchArgs& b, int precision, int n_state, int kind, int grid, cudaStream_t s);
+// The same per form (stage_plain.cu, stage_mixed.cu, stage_delta.cu).
+template <int P> cudaError_t launch_stage_form(const StageArgs& a, int n_state, int order, int kind, cudaStream_t s);
+template <int P> cudaError_t launch_batch_form(const BatchArgs& b, int n_state, int kind, int grid, cudaStream_t s);
+template <int P> cudaError_t prepare_batch_form();
 cudaError_t prepare_batch_kernels(int precision);
 int batch_ctas_per_sm(int precision);
 cudaError_t launch_lism_init(const GridGeom& g, const double* lism, uint64_t seed, double pert,
@@ -401,6 +400,5 @@ cudaError_t launch_chlld_batch(int64_t n, int n_state, int n_disc, int precision
 cudaError_t launch_chlld_q_batch(int64_t n, int n_state, int n_disc, bool ydar, const double* normals,
                                  const double* w, const double* q1, const double* q2, double* konvect,
                                  double* qqq, double* speeds, int32_t* flags, cudaStream_t s);
-int stage_fp64_smem_bytes();
 
 }  // namespace sb
