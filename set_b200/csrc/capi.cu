@@ -122,8 +122,11 @@ int shape_index(int precision, int kind) {
 
 }  // namespace
 
-// z extent of one CTA's march: balances wave quantisation against the per-chunk prologue
-// (4 plane loads + 1 z face, costed as ~1.5 plane iterations).
+// z extent of one CTA's march: balances wave quantisation against what a chunk costs beside its
+// planes (launch, four planes loaded, the last z face and update: about three intervals of the
+// march, measured 16 us beside 5.5 us a plane on grids of one wave).  Chunks go down to one plane:
+// a small grid has too few columns for the SMs, and shorter marches cost more work but less time
+// (32^3 a stage 56 us at 8 planes, 22 us at one; 64^3 59 us at 8, 49 us at 6).
 int sb::choose_lz(const GridGeom& g, int sm_count, int precision, int kind) {
     const TileShape ts = tile_shape(precision, kind);
     const long long cols = (long long)((g.nx + kTileX - 1) / kTileX) * ((g.ny + ts.ty - 1) / ts.ty);
@@ -131,11 +134,11 @@ int sb::choose_lz(const GridGeom& g, int sm_count, int precision, int kind) {
     const int nz = plane_end(g) - plane_begin(g);   // planes the stage kernels update
     double best = 1e300;
     int best_lz = nz;
-    for (int c = 1; c <= std::max(1, nz / 8); c++) {
+    for (int c = 1; c <= nz; c++) {
         const int lz = (nz + c - 1) / c;
         const long long ctas = cols * ((nz + lz - 1) / lz);
         const long long waves = (ctas + slots - 1) / slots;
-        const double cost = (double)waves * (lz + 1.5);
+        const double cost = (double)waves * (lz + 3);
         if (cost < best - 1e-9) {
             best = cost;
             best_lz = lz;

@@ -9,20 +9,20 @@
 namespace sb {
 
 // Column tile of the stage kernels: kTileX x ty cells marched along z by `threads` threads, one warp
-// per tile row and one for the tile's edges, `ctas_per_sm` resident per SM, `boxes` staged planes.
+// per tile row and one for the tile's edges, `ctas_per_sm` resident per SM.
 // The plain and delta forms' FP64 ring limits the tile to 11 rows (223 KB of shared memory; 12
 // warps of 168 registers: 16 warps of 128 with 10 rows spill, 2.65 / 2.74 against 2.31 / 2.44 ms a
 // stage at 256^3 when it was tried).  The mixed form's FP32 ring leaves room for 15 rows: 16 warps
 // of 128 registers and the smallest halo (1.43 cells staged per cell; 384^3, stage 1 / 2: 4.82 /
-// 5.58 ms against 5.32 / 6.12 with 11 rows and 12 warps).  Its two staged boxes would fit, but leave
+// 5.58 ms against 5.32 / 6.12 with 11 rows and 12 warps).  A second staged box would fit, but leaves
 // 18 KB of L1 for the second stage's loads: 6.32 against 5.58 ms.
 constexpr int kTileX = 32;
 struct TileShape {
-    int ty, threads, ctas_per_sm, boxes;
+    int ty, threads, ctas_per_sm;
 };
 SB_HD constexpr TileShape tile_shape(int precision, int kind) {
     (void)kind;
-    return precision == 1 ? TileShape{15, 512, 1, 1} : TileShape{11, 384, 1, 1};
+    return precision == 1 ? TileShape{15, 512, 1} : TileShape{11, 384, 1};
 }
 // The tile_shape kind every batch launch uses.
 constexpr int kBatchKind = 1;

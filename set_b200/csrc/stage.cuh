@@ -66,13 +66,12 @@ template <int P, int SK> struct Tile {   // SK: the launch kind of tile_shape
     static constexpr int NC = TX * TY;
     static constexpr int HX = TX + 4, HY = TY + 4, PLANE = HX * HY;
     static constexpr int NYF = TX * (TY + 1);        // y faces
-    // staging boxes (plane copies in flight)
     using RG = typename Types<P>::Ring;
     using FT = typename Types<P>::Flux;
-    static constexpr int kStage = 8 * PLANE * (int)sizeof(double);
-    static constexpr int kRest = 128 + RING * 8 * PLANE * (int)sizeof(RG) + 2 * 8 * (NYF + TY) * (int)sizeof(FT);
-    static constexpr int NSTG = tile_shape(P, SK).boxes;
-    static constexpr int kSmem = kRest + NSTG * kStage;
+    // dynamic shared memory: alignment slack, staged box (FP64), primitive ring, and the exchanged y
+    // and east x fluxes (two buffers each)
+    static constexpr int kSmem = 128 + 8 * PLANE * (int)sizeof(double) + RING * 8 * PLANE * (int)sizeof(RG) +
+                                 2 * 8 * (NYF + TY) * (int)sizeof(FT);
     static_assert(TX == 32, "one lane per tile column");
     static_assert(NT == 32 * (TY + 1), "one warp per tile row and one for the edges");
     static_assert(TY <= 32, "one lane per row for the east faces");
@@ -112,16 +111,19 @@ __device__ __forceinline__ void fetch_prim64(const StageArgs& A, int i, int j, i
     }
 }
 
-// Loads the cells c0, c0 + step, ... < c1 of plane kk (with halo) of the tile starting at (i0, j0)
-// as primitives into `dst`.
+// Loads cells n0, n0 + step, ... < n1 of the planes from kk on (with halo; cell n is cell n % PLANE of
+// plane kk + n / PLANE) of the tile starting at (i0, j0) as primitives into their ring slots.
 template <int P, int SK, typename RT>
-__device__ __forceinline__ void load_plane(const StageArgs& A, RT* dst, int i0, int j0, int kk, int c0, int step,
-                                           int c1) {
+__device__ __forceinline__ void load_planes(const StageArgs& A, RT* ring, int i0, int j0, int kk, int n1, int n0,
+                                            int step) {
     constexpr int HX = Tile<P, SK>::HX, PLANE = Tile<P, SK>::PLANE;
-    for (int c = c0; c < c1; c += step) {
+#pragma unroll 2
+    for (int n = n0; n < n1; n += step) {
+        const int k = kk + n / PLANE, c = n % PLANE;
         const int cx = c % HX, cy = c / HX;
+        RT* dst = ring + ring_slot(k) * 8 * PLANE;
         double q[8];
-        fetch_prim64<P != 1, P == 0>(A, i0 - 2 + cx, j0 - 2 + cy, kk, q);
+        fetch_prim64<P != 1, P == 0>(A, i0 - 2 + cx, j0 - 2 + cy, k, q);
 #pragma unroll
         for (int v = 0; v < 8; v++) dst[v * PLANE + c] = (RT)q[v];
     }
@@ -407,7 +409,7 @@ __device__ __forceinline__ void update_cell(const StageArgs& A, const CellState<
 // the solve's clock.  Called by the single-solve kernel (one tile per CTA) and by the batch
 // kernel (tiles of many solves drawn from a work queue); every CTA-wide barrier is reached by all
 // threads, and the function ends with one so a CTA may run the next tile immediately.
-// `phases` holds the parity of the next wait on each staging box's barrier (bit b: bar[b]) and `tma_dead` is set once a plane copy did not
+// `phase` is the parity of the next wait on the staging box's barrier and `tma_dead` is set once a plane copy did not
 // land within both bounded waits (the thread then reads its planes with plain loads); both are
 // per thread and carried across the tiles a CTA runs.
 //
@@ -432,21 +434,21 @@ __device__ __forceinline__ void update_cell(const StageArgs& A, const CellState<
 // instruction fetch), the solver unchanged.
 template <int P, int NSTATE, int ORDER, int KIND, int SK, int ND>
 __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int bz, unsigned total_tiles,
-                                         unsigned long long* bar, unsigned& phases, bool& tma_dead) {
+                                         unsigned long long* bar, unsigned& phase, bool& tma_dead) {
     using RG = typename Types<P>::Ring;
     using FT = typename Types<P>::Flux;
     using RT = typename Types<P>::Math;
     using C = Tile<P, SK>;
     constexpr bool WANT_DT = KIND == 0;   // the first stage's faces give the next step's dt
     constexpr int TX = C::TX, TY = C::TY, NC = C::NC, NT = C::NT, HX = C::HX, PLANE = C::PLANE;
-    constexpr int NYF = C::NYF, NSTG = C::NSTG;
+    constexpr int NYF = C::NYF;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    // NSTG staged conserved boxes [8][PLANE]; tensor copies land on a 128-byte aligned address.  The
+    // [8][PLANE] staged conserved box; tensor copies land on a 128-byte aligned address.  The
     // alignment pad is an offset from the shared array itself, so every pointer below stays in
     // the shared address space (shared loads and stores with 32-bit addresses, not generic ones).
     const unsigned pad = (128u - (smem_u32(smem_raw) & 127u)) & 127u;
     double* stg = reinterpret_cast<double*>(smem_raw + pad);
-    RG* ring = reinterpret_cast<RG*>(stg + NSTG * 8 * PLANE);
+    RG* ring = reinterpret_cast<RG*>(stg + 8 * PLANE);
     FT* fy = reinterpret_cast<FT*>(ring + RING * 8 * PLANE);   // [2][8][NYF]: y fluxes of plane k at k & 1
     FT* fe = fy + 2 * 8 * NYF;                                  // [2][8][TY]: east x fluxes
     __shared__ double red[NT / 32];
@@ -470,16 +472,14 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int
     double rate = 0.0;   // max over this thread's real faces of max(|SL|,|SR|)/dist
     unsigned n_recon = 0, n_wave = 0, n_redo = 0, n_tmo = 0;
 
-    // ---- plane staging.  Plane kk enters ring slot kk & 3.  With a tensor map, the copies of the
-    // next NSTG planes are in flight while the faces and the update of an interval run; the last
-    // copy issued is plane k1+1.
+    // ---- plane staging.  Plane kk enters ring slot kk & 3.  With a tensor map, the copy of the
+    // next plane is in flight while the faces and the update of an interval run; the last copy
+    // issued is plane k1+1.
     const bool use_tma = A.tm_in != nullptr && !tma_dead;
     constexpr unsigned kPlaneBytes = 8u * PLANE * sizeof(double);
-    const int kz_first = k0 - 2, kz_last = k1 + 1;
-    auto box = [&](int kk) { return NSTG == 2 ? (kk - kz_first) & 1 : 0; };
+    const int kz_last = k1 + 1;
     auto issue_copy = [&](int kk) {
-        tma_plane(stg + box(kk) * 8 * PLANE, A.tm_in, i0 - 2, j0 - 2, min(max(kk, 0), g.nz - 1), kPlaneBytes,
-                  bar + box(kk));
+        tma_plane(stg, A.tm_in, i0 - 2, j0 - 2, min(max(kk, 0), g.nz - 1), kPlaneBytes, bar);
     };
     // Converts plane kk for the cells c0, c0 + step, ... < c1 of this thread.
     auto take_plane = [&](int kk, int c0, int step, int c1) {
@@ -488,26 +488,28 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int
             // A wait that runs out is counted (SETB_ETIMEOUT), then the copy gets a second bounded
             // wait to land before the box is read; a copy that never lands switches this thread to
             // plain loads (and thread 0 stops issuing copies), so no read races a late copy.
-            const int b = box(kk);
-            const unsigned parity = (phases >> b) & 1u;
-            bool ok = mbar_wait_bounded(bar + b, parity, A.copy_wait);
+            bool ok = mbar_wait_bounded(bar, phase, A.copy_wait);
             if (!ok) {
                 n_tmo++;
-                ok = mbar_wait_bounded(bar + b, parity, kCopyWaitCycles);
+                ok = mbar_wait_bounded(bar, phase, kCopyWaitCycles);
             }
-            phases ^= 1u << b;
-            if (ok) convert_plane<P, SK, RG>(A, stg + b * 8 * PLANE, slot, i0, j0, c0, step, c1);
+            phase ^= 1u;
+            if (ok) convert_plane<P, SK, RG>(A, stg, slot, i0, j0, c0, step, c1);
             else tma_dead = true;
         }
-        if (!use_tma || tma_dead) load_plane<P, SK, RG>(A, slot, i0, j0, kk, c0, step, c1);
+        if (!use_tma || tma_dead) load_planes<P, SK, RG>(A, ring, i0, j0, kk, c1, c0, step);
         __syncthreads();
-        if (use_tma && !tma_dead && t == 0 && kk + NSTG <= kz_last) issue_copy(kk + NSTG);
+        if (use_tma && !tma_dead && t == 0 && kk < kz_last) issue_copy(kk + 1);
     };
-    if (use_tma && t == 0) {
-        for (int b = 0; b < NSTG; b++) issue_copy(kz_first + b);
-    }
-#pragma unroll 1
-    for (int kk = kz_first; kk <= k0 + 1; kk++) take_plane(kk, t, NT, PLANE);
+    // The first four planes come by plain loads, all in flight together, while the first copy (plane
+    // k0+2) runs: the values are the same, and four copies one after the other through the staging
+    // box would take four latencies (32^3 a stage: 22 -> 20 us).
+    if (use_tma && t == 0) issue_copy(k0 + 2);
+    // a negative wait limit is one check of the tile's first copy right behind its issue (by the time
+    // the faces are done it has landed)
+    if (use_tma && A.copy_wait < 0 && !mbar_test_wait(bar, phase)) n_tmo++;
+    load_planes<P, SK, RG>(A, ring, i0, j0, k0 - 2, 4 * PLANE, t, NT);
+    __syncthreads();
 
     // whether this thread's column crosses the source sphere (x^2 + y^2 < r_src^2)
     bool col_src;
@@ -824,16 +826,13 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int
 
 template <int P, int NSTATE, int ORDER, int KIND, int ND>
 __global__ void __launch_bounds__(Tile<P, KIND>::NT, Tile<P, KIND>::MINB) stage_kernel(const StageArgs A) {
-    __shared__ __align__(8) unsigned long long bar[2];
-    if (threadIdx.x == 0) {
-        mbar_init(bar);
-        mbar_init(bar + 1);
-    }
+    __shared__ __align__(8) unsigned long long bar;
+    if (threadIdx.x == 0) mbar_init(&bar);
     __syncthreads();
-    unsigned phases = 0;
+    unsigned phase = 0;
     bool tma_dead = false;
     run_tile<P, NSTATE, ORDER, KIND, KIND, ND>(A, blockIdx.x, blockIdx.y, blockIdx.z,
-                                                         gridDim.x * gridDim.y * gridDim.z, bar, phases, tma_dead);
+                                                         gridDim.x * gridDim.y * gridDim.z, &bar, phase, tma_dead);
 }
 
 // Persistent batch kernel: each CTA takes tiles from the work queue until it is empty; the
@@ -844,14 +843,11 @@ template <int P, int NSTATE, int ORDER, int KIND>
 __global__ void __launch_bounds__(Tile<P, kBatchKind>::NT, Tile<P, kBatchKind>::MINB) batch_stage_kernel(const BatchArgs B) {
     __shared__ __align__(16) StageArgs As;
     __shared__ int4 it;
-    __shared__ __align__(8) unsigned long long bar[2];
+    __shared__ __align__(8) unsigned long long bar;
     constexpr int WORDS = sizeof(StageArgs) / sizeof(unsigned long long);
     static_assert(sizeof(StageArgs) % sizeof(unsigned long long) == 0, "StageArgs must be 8-byte granular");
-    if (threadIdx.x == 0) {
-        mbar_init(bar);
-        mbar_init(bar + 1);
-    }
-    unsigned phases = 0;   // the same in every thread
+    if (threadIdx.x == 0) mbar_init(&bar);
+    unsigned phase = 0;   // the same in every thread
     bool tma_dead = false;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -865,22 +861,15 @@ __global__ void __launch_bounds__(Tile<P, kBatchKind>::NT, Tile<P, kBatchKind>::
         unsigned long long* dst = reinterpret_cast<unsigned long long*>(&As);
         for (int q = threadIdx.x; q < WORDS; q += Tile<P, kBatchKind>::NT) dst[q] = src[q];
         __syncthreads();
-        run_tile<P, NSTATE, ORDER, KIND, kBatchKind, 2>(As, w.y, w.z, w.w, As.total_tiles, bar,
-                                                                  phases, tma_dead);
+        run_tile<P, NSTATE, ORDER, KIND, kBatchKind, 2>(As, w.y, w.z, w.w, As.total_tiles, &bar,
+                                                                  phase, tma_dead);
     }
-}
-
-// Dynamic shared memory: alignment slack, staged boxes (FP64), primitive ring, and the exchanged y
-// and east x fluxes (two buffers each).
-template <int P, int SK>
-constexpr int smem_bytes() {
-    return Tile<P, SK>::kSmem;
 }
 
 template <int P, int NSTATE, int ORDER, int KIND, int ND>
 cudaError_t launch_nd(const StageArgs& a, cudaStream_t s) {
     auto kern = stage_kernel<P, NSTATE, ORDER, KIND, ND>;
-    const int smem = smem_bytes<P, KIND>();
+    const int smem = Tile<P, KIND>::kSmem;
     // The dynamic shared-memory opt-in is a per-device attribute of the kernel: set it once per
     // device ordinal (a bit per device, atomically; two threads that both set it set the same
     // value), and on every launch for ordinals beyond the mask.
@@ -919,17 +908,17 @@ cudaError_t launch_n(const StageArgs& a, int order, int kind, cudaStream_t s) {
 template <int P, int NSTATE>
 cudaError_t batch_attr() {
     cudaError_t e = cudaFuncSetAttribute(batch_stage_kernel<P, NSTATE, 2, 0>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<P, kBatchKind>());
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<P, kBatchKind>::kSmem);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(batch_stage_kernel<P, NSTATE, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                smem_bytes<P, kBatchKind>());
+                                Tile<P, kBatchKind>::kSmem);
 }
 
 template <int P, int NSTATE>
 void launch_batch_n(const BatchArgs& b, int kind, int grid, cudaStream_t s) {
     constexpr int NT = Tile<P, kBatchKind>::NT;
-    if (kind == 0) batch_stage_kernel<P, NSTATE, 2, 0><<<grid, NT, smem_bytes<P, kBatchKind>(), s>>>(b);
-    else batch_stage_kernel<P, NSTATE, 2, 1><<<grid, NT, smem_bytes<P, kBatchKind>(), s>>>(b);
+    if (kind == 0) batch_stage_kernel<P, NSTATE, 2, 0><<<grid, NT, Tile<P, kBatchKind>::kSmem, s>>>(b);
+    else batch_stage_kernel<P, NSTATE, 2, 1><<<grid, NT, Tile<P, kBatchKind>::kSmem, s>>>(b);
 }
 
 }  // namespace
