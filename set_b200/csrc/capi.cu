@@ -575,7 +575,8 @@ int32_t setb_init_cartesian_lism(setb_handle** out, const setb_cart_desc* d, con
 namespace {
 // Enqueues nsteps steps.  When ev is non-null, ev[0..2*nsteps] are recorded before the first
 // launch and after every launch (Euler: ev[2s+1] == ev[2s+2] bracket nothing).
-// Face-list steps: same stage sequence and events as the Cartesian path, three launches per stage.
+// Face-list steps: same stage sequence and events as the Cartesian path, two launches per stage (and
+// the primitive pass before the first).
 int enqueue_fl_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaEvent_t* ev) {
     if (o->precision != 0) return SETB_EINVAL;
     h->comp_clean = false;
@@ -584,12 +585,12 @@ int enqueue_fl_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cu
         double* U = h->buf[h->cur];
         double* W = h->buf[1 - h->cur];
         if (o->scheme == 2) {
-            SB_TRY(fl_launch_stage(h->fl, U, nullptr, W, h->g.vs, h->clk, h->st, o, 0, true, false, h->stream));
+            SB_TRY(fl_launch_stage(h->fl, U, nullptr, W, h->g.vs, h->clk, h->st, o, 0, true, false, s == 0, true, h->stream));
             if (ev) SB_TRY(cudaEventRecord(ev[2 * s + 1], h->stream));
-            SB_TRY(fl_launch_stage(h->fl, W, U, U, h->g.vs, h->clk, h->st, o, 1, false, true, h->stream));
+            SB_TRY(fl_launch_stage(h->fl, W, U, U, h->g.vs, h->clk, h->st, o, 1, false, true, false, s + 1 < nsteps, h->stream));
             if (ev) SB_TRY(cudaEventRecord(ev[2 * s + 2], h->stream));
         } else {
-            SB_TRY(fl_launch_stage(h->fl, U, nullptr, W, h->g.vs, h->clk, h->st, o, 0, true, true, h->stream));
+            SB_TRY(fl_launch_stage(h->fl, U, nullptr, W, h->g.vs, h->clk, h->st, o, 0, true, true, s == 0, s + 1 < nsteps, h->stream));
             if (ev) {
                 SB_TRY(cudaEventRecord(ev[2 * s + 1], h->stream));
                 SB_TRY(cudaEventRecord(ev[2 * s + 2], h->stream));

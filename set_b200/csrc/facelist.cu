@@ -5,12 +5,13 @@
 // (CUF_MGD_grans_RK2, :243-440) computes each face's flux once into Gran_POTOK and a cell kernel
 // (CUF_MGD_cell_RK2, :561-794) sums the fluxes of its faces with the owner sign.  This file keeps
 // that structure, B200-side:
-//   * the cell state is conserved SoA FP64 (coalesced in the cell kernel); each stage starts
-//     with a pass that writes the primitive state cell-major (8 doubles = 64 B per cell), so a
-//     face gathers a cell with four 16-byte loads;
-//   * per-face geometry the face kernel needs (the four TVD distances, the reference's "skip"
-//     rule) is derived once at set-up, in the same FP64 arithmetic as the reference's per-step
-//     computation, so the stage kernels read it instead of recomputing it from cell centres;
+//   * the cell state is conserved SoA FP64 (coalesced in the cell kernel); the primitive state is
+//     kept beside it cell-major (8 doubles = 64 B per cell), so a face gathers a cell with four
+//     16-byte loads; a pass of its own forms it for the first stage of a call, the cell kernel
+//     leaves it for every later one;
+//   * per-face geometry the face kernel needs (the slope weights of the TVD distances, the
+//     reference's "skip" rule, the owner sign) is derived once at set-up in FP64, so the stage
+//     kernels read it instead of recomputing it from cell centres;
 //   * the face kernel reduces the dt candidate with warp shuffles and one atomicMin per block;
 //     the cell kernel's last block rolls the lagged-dt clock on the device, so a run of steps
 //     needs no host round trip;
@@ -29,32 +30,41 @@
 
 #include "setb200.h"
 #include "setb_internal.cuh"
+#include "riemann_fp64.cuh"
 
 namespace sb {
 
-struct FaceListDev {
+// What the kernels read (passed by value).
+struct FlView {
     int64_t n_cell = 0, n_gran = 0;
     // cells
     double* cell_center = nullptr;   // [N][3]
-    double* cell_volume = nullptr;   // [N]
-    int32_t* cell_gran = nullptr;    // [N][6], 1-based face numbers, 0 = none
-    unsigned char* cell_flag = nullptr;   // bit 0: frozen (not updated)
+    double* inv_volume = nullptr;    // [N] 1 / volume
+    int32_t* cell_gran = nullptr;    // [N][6]: +-(face + 1), + where the cell is the face's first
+                                     // neighbour; 0 = none
+    unsigned char* cell_flag = nullptr;   // kFrozen, kSource
     // faces
-    double* normal = nullptr;        // [G][3]
-    double* square = nullptr;        // [G]
-    double* geo = nullptr;           // [G][4]: dist = |c_face - c_s1|, df2, dff1, dff2
-    int32_t* nb = nullptr;           // [G][2], 1-based, -1 = none
-    int32_t* nbt = nullptr;          // [G][2], 1-based, -1 = none
-    int32_t* type = nullptr;         // [G]: 0 = skipped, else the reference's face type 1..5,
-                                     // plus kLaxFace on the near-axis faces of physics 1
+    double* normal = nullptr;        // [G][4]: normal, area
+    double* geo = nullptr;           // [G][4]: dist = |c_face - c_s1|, and the weights of the face
+                                     // values' slopes (fl_face_kernel)
+    int32_t* nb = nullptr;           // [G][4]: neighbours 1, 2 (a ghost face: 1 again) and the TVD cells
+                                     // (both -1 where the face is first order), 0-based
+    int32_t* type = nullptr;         // [G]: 0 = skipped, else the reference's face type 1..5
+                                     // (kInner: an interior type-2 face), plus kLaxFace on the
+                                     // near-axis faces of physics 1
     // work
-    double* prim = nullptr;          // [N][8] primitive state of the stage input
-    double* flux = nullptr;          // [G][8] face flux * area (persistent)
+    double* prim = nullptr;          // [N][8] primitive state of the stage input, field as b = B / sqrt(4 pi)
+    double* flux = nullptr;          // [G+1][8] face flux * area (persistent), field fluxes in units of b;
+                                     // the last row stays zero (a cell's missing faces)
     GridGeom src{};                  // source-sphere parameters (r_src 0 = none)
-    int physics = 0;                 // 0: 3D MHD; 1: the reference's axisymmetric hydro update
     double* hatom = nullptr;         // physics 1: [N][8] H-atom fluids (Cell_par columns 9..16)
     int powell = 0;                  // physics 0: div-B terms (0 off, 1 momentum + induction, 2 + energy)
-    double* divb = nullptr;          // powell: [G] div-B face flux * area, Gran_POTOK(9) (persistent)
+    double* divb = nullptr;          // powell: [G+1] div-B face flux * area, Gran_POTOK(9) (persistent)
+};
+
+struct FaceListDev {
+    FlView v;
+    int physics = 0;                 // 0: 3D MHD; 1: the reference's axisymmetric hydro update
     // locality order: device cell d holds the caller's cell perm[d] (both 0-based)
     std::vector<int32_t> perm;
 };
@@ -62,7 +72,9 @@ struct FaceListDev {
 namespace {
 
 constexpr int kFaceThreads = 128, kCellThreads = 256, kPrimThreads = 256;
+constexpr int kInner = 6;     // face type: a type-2 face with a second neighbour
 constexpr int kLaxFace = 8;   // face-type bit: the reference's Lax flux on near-axis faces
+constexpr int kFrozen = 1, kSource = 2;   // cell flags: not updated; inside the source sphere
 
 double norm3(const double* x) {
     return std::sqrt((x[0] * x[0] + x[1] * x[1]) + x[2] * x[2]);
@@ -76,30 +88,29 @@ cudaError_t upload(T** dst, const T* src, size_t n, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------------------ kernels
+__device__ __forceinline__ void store_prim(double* P, int64_t c, const double* q) {
+    double2* p2 = reinterpret_cast<double2*>(P + 8 * c);
+#pragma unroll
+    for (int v = 0; v < 4; v++) p2[v] = make_double2(q[2 * v], q[2 * v + 1]);
+}
+
+// Primitive state of the first stage of a call (later stages get theirs from the cell kernel).
 __global__ void fl_prim_kernel(int64_t n, const double* __restrict__ U, int64_t vs, double* __restrict__ P) {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
         double u8[8], q[8], ke, me;
 #pragma unroll
         for (int v = 0; v < 8; v++) u8[v] = U[v * vs + c];
-        prim_from_cons(u8, q, ke, me);
-        double2* p2 = reinterpret_cast<double2*>(P + 8 * c);
-#pragma unroll
-        for (int v = 0; v < 4; v++) p2[v] = make_double2(q[2 * v], q[2 * v + 1]);
+        prim_from_cons<true, true>(u8, q, ke, me);
+        store_prim(P, c, q);
     }
 }
 
-// Solvers.f90:141-150 at y = 0: linear(x1,t1,x2,t2,x3,t3,0) = minmod of the two one-sided
-// slopes times (0 - x2), plus t2, with ra = 1/(x1 - x2) and rb = 1/(x2 - x3) (geometry, formed
-// once per face): the slopes' divisions become multiplications, one rounding from the reference.
-__device__ __forceinline__ double linear_rcp(double ra, double t1, double x2, double t2, double rb, double t3) {
-    const double d = minmod(dmul(dsub(t1, t2), ra), dmul(dsub(t2, t3), rb));
-    return dadd(dmul(d, dsub(0.0, x2)), t2);
-}
-
+// The first NV (even) components of a cell's primitive state.
+template <int NV = 8>
 __device__ __forceinline__ void load_prim(const double* P, int64_t c, double* q) {
     const double2* p2 = reinterpret_cast<const double2*>(P + 8 * c);
 #pragma unroll
-    for (int v = 0; v < 4; v++) {
+    for (int v = 0; v < NV / 2; v++) {
         const double2 d = __ldg(p2 + v);
         q[2 * v] = d.x;
         q[2 * v + 1] = d.y;
@@ -108,35 +119,36 @@ __device__ __forceinline__ void load_prim(const double* P, int64_t c, double* q)
 
 // Source_MK (SET_Fortran_Cuda_MHD/cuf_kernel.cuf:215-288): charge-exchange momentum (x, y) and
 // energy sources against two H-atom fluids (rho, u, v, T per fluid in h[0..3], h[4..7]).  The
-// reference's default-real literals enter as their single-precision values.
+// reference's default-real literals enter as their single-precision values.  Common denominators are
+// reciprocals (rounding only): the cell kernel is a chain of dependent FP64 operations.
 __device__ __forceinline__ void source_mk(const double* q, const double* h, double* out) {
     const double pi = 3.141592653589793;
     const double rho = q[0], u = q[1], v = q[2], p = q[4];
     const double small = (double)0.0000001f;
-    const double c_m = __ddiv_rn(64.0, dmul(9.0, pi)), c_u = __ddiv_rn(4.0, pi);
+    const double c_m = 64.0 / (9.0 * pi), c_u = 4.0 / pi;
     const double c_s = (double)0.1307345665f;
     const double c_n = (double)(3.0f / 0.4326569f);
+    const double tp = p * rs_rcp(rho);   // p / rho
     double s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-        double rH = h[4 * k], uH = h[4 * k + 1], vH = h[4 * k + 2];
-        double pH = dmul(dmul(0.5, h[4 * k + 3]), rH);
+        double rH = h[4 * k], tH = h[4 * k + 3];   // 2 pH / rH = T
+        const double uH = h[4 * k + 1], vH = h[4 * k + 2];
         if (rH < small) {
             rH = small;
-            pH = 0.0;
+            tH = 0.0;
         }
-        const double du = dsub(u, uH), dv = dsub(v, vH);
-        const double th = dadd(__ddiv_rn(p, rho), __ddiv_rn(dmul(2.0, pH), rH));
-        const double d2 = dadd(dmul(du, du), dmul(dv, dv));
-        const double UM = sqrt(dadd(d2, dmul(c_m, th)));
-        const double UH = sqrt(dadd(d2, dmul(c_u, th)));
-        const double lg = dsub(1.0, dmul(c_s, log(UM)));
-        const double nu = dmul(dmul(dmul(rho, rH), UM), dmul(lg, lg));
-        const double cn = dmul(c_n, nu);
-        s1 = dadd(s1, dmul(cn, dsub(uH, u)));
-        s2 = dadd(s2, dmul(cn, dsub(vH, v)));
-        const double ke = __ddiv_rn(dsub(dsub(dadd(dmul(uH, uH), dmul(vH, vH)), dmul(u, u)), dmul(v, v)), 2.0);
-        s3 = dadd(s3, dmul(cn, dadd(ke, dmul(__ddiv_rn(UH, UM), dsub(__ddiv_rn(dmul(2.0, pH), rH), __ddiv_rn(p, rho))))));
+        const double du = u - uH, dv = v - vH;
+        const double th = tp + tH;
+        const double d2 = fma(dv, dv, du * du);
+        const double um2 = fma(c_m, th, d2), uh2 = fma(c_u, th, d2);
+        const double iUM = rs_rsqrt(um2), UM = um2 * iUM, UH = over_sqrt(uh2, uh2);
+        const double lg = fma(-0.5 * c_s, log(um2), 1.0);
+        const double cn = c_n * ((rho * rH * UM) * (lg * lg));
+        s1 = fma(cn, uH - u, s1);
+        s2 = fma(cn, vH - v, s2);
+        const double ke = 0.5 * (fma(vH, vH, uH * uH) - fma(v, v, u * u));
+        s3 = fma(cn, fma(UH * iUM, tH - tp, ke), s3);
     }
     out[0] = s1;
     out[1] = s2;
@@ -144,74 +156,79 @@ __device__ __forceinline__ void source_mk(const double* q, const double* h, doub
 }
 
 // The reference's live cell update (cuf_solvers.cuf:561-794): 2D axisymmetric hydro about the x
-// axis with radius rr(2) = y, w = B = 0, charge exchange, p floor and the near-axis v clamp, in
-// the reference's operation order on the primitive state.  Writes the conserved result to un;
-// returns 1 for a non-positive density (un = the stage input), 2 when the p floor applied.
+// axis with radius rr(2) = y, w = B = 0, charge exchange, p floor and the near-axis v clamp.  q: the
+// stage input's primitive state; writes the conserved result to un; returns 1 for a non-positive
+// density (un = the stage input), 2 when the p floor applied.
 template <int KIND>
 __device__ __forceinline__ int axisym_update(const double* Uin, const double* Ubase, int64_t vs, int64_t c,
-                                             const double* pot, double vol, double x, double y, const double* h,
-                                             double t, double* un) {
-    const double g = kGamma, gm1 = dsub(kGamma, 1.0);
-    double u8[8], q[8], q2[8], ke, me, source[3];
+                                             const double* q, const double* pot, double ivol, double x, double y,
+                                             const double* h, double t, double* un) {
+    double u8[8], source[3];
 #pragma unroll
     for (int v = 0; v < 8; v++) u8[v] = Uin[v * vs + c];
-    prim_from_cons_exact(u8, q);
+    double b8[8];   // the base state of the sum: itself, or Heun stage 2's U^n (energies without field)
     if (KIND == 1) {
-        double b8[8];
 #pragma unroll
         for (int v = 0; v < 8; v++) b8[v] = Ubase[v * vs + c];
-        prim_from_cons_exact(b8, q2);
+        b8[4] -= (0.5 * kInvSpi4 * kInvSpi4) * fma(b8[7], b8[7], fma(b8[6], b8[6], b8[5] * b8[5]));
     }
-    (void)ke;
-    (void)me;
     source_mk(q, h, source);
-    const double nq = sqrt(dadd(dadd(dmul(q[1], q[1]), dmul(q[2], q[2])), dmul(q[3], q[3])));
-    const double e1 = dadd(__ddiv_rn(q[4], gm1), dmul(dmul(0.5, q[0]), dmul(nq, nq)));
-    const double X = dadd(__ddiv_rn(dmul(g, q[4]), gm1), dmul(dmul(q[0], dadd(dmul(q[1], q[1]), dmul(q[2], q[2]))), 0.5));
-    const double geo_e = __ddiv_rn(dmul(dmul(t, q[2]), X), y);
-    const double div0 = dadd(__ddiv_rn(pot[0], vol), __ddiv_rn(dmul(q[0], q[2]), y));
-    double ro3;
-    if (KIND == 0) ro3 = dsub(q[0], dmul(t, div0));
-    else ro3 = dmul(0.5, dsub(dadd(q2[0], q[0]), dmul(t, div0)));
+    const double iy = rs_rcp(y);
+    const double uv2 = fma(q[2], q[2], q[1] * q[1]);
+    const double e1 = fma(0.5 * q[0], fma(q[3], q[3], uv2), kInvG1 * q[4]);
+    const double X = fma(0.5 * q[0], uv2, (kGamma * kInvG1) * q[4]);
+    const double rv = q[0] * q[2] * iy;   // rho v / y
+    const double d0 = fma(pot[0], ivol, rv), d1 = fma(pot[1], ivol, fma(rv, q[1], -source[0]));
+    const double d2 = fma(pot[2], ivol, fma(rv, q[2], -source[1]));
+    const double d4 = fma(pot[4], ivol, fma(q[2] * iy, X, -source[2]));
+    double ro3, mx, my, e3;
+    if (KIND == 0) {
+        ro3 = fma(-t, d0, u8[0]);
+        mx = fma(-t, d1, u8[1]);
+        my = fma(-t, d2, u8[2]);
+        e3 = fma(-t, d4, e1);
+    } else {
+        ro3 = 0.5 * fma(-t, d0, b8[0] + u8[0]);
+        mx = 0.5 * fma(-t, d1, b8[1] + u8[1]);
+        my = 0.5 * fma(-t, d2, b8[2] + u8[2]);
+        e3 = 0.5 * fma(-t, d4, b8[4] + e1);
+    }
     if (!(ro3 > 0.0)) {
 #pragma unroll
         for (int v = 0; v < 8; v++) un[v] = u8[v];
         return 1;
     }
-    const double g1 = __ddiv_rn(dmul(t, pot[1]), vol), g2 = __ddiv_rn(dmul(t, pot[2]), vol);
-    const double g4 = __ddiv_rn(dmul(t, pot[4]), vol);
-    const double a1 = __ddiv_rn(dmul(dmul(dmul(t, q[0]), q[1]), q[2]), y);
-    const double a2 = __ddiv_rn(dmul(dmul(dmul(t, q[0]), q[2]), q[2]), y);
-    double u3, v3, p3;
-    if (KIND == 0) {
-        u3 = __ddiv_rn(dsub(dadd(dsub(dmul(q[0], q[1]), g1), dmul(t, source[0])), a1), ro3);
-        v3 = __ddiv_rn(dsub(dadd(dsub(dmul(q[0], q[2]), g2), dmul(t, source[1])), a2), ro3);
-        p3 = dmul(dsub(dsub(dadd(dsub(e1, g4), dmul(t, source[2])), geo_e),
-                       dmul(dmul(0.5, ro3), dadd(dadd(dmul(u3, u3), dmul(v3, v3)), 0.0))),
-                  gm1);
-    } else {
-        const double nq2 = sqrt(dadd(dadd(dmul(q2[1], q2[1]), dmul(q2[2], q2[2])), dmul(q2[3], q2[3])));
-        const double e2 = dadd(__ddiv_rn(q2[4], gm1), dmul(dmul(0.5, q2[0]), dmul(nq2, nq2)));
-        u3 = __ddiv_rn(dmul(0.5, dsub(dadd(dsub(dadd(dmul(q2[0], q2[1]), dmul(q[0], q[1])), g1), dmul(t, source[0])), a1)), ro3);
-        v3 = __ddiv_rn(dmul(0.5, dsub(dadd(dsub(dadd(dmul(q2[0], q2[2]), dmul(q[0], q[2])), g2), dmul(t, source[1])), a2)), ro3);
-        p3 = dmul(dsub(dmul(0.5, dsub(dadd(dsub(dadd(e2, e1), g4), dmul(t, source[2])), geo_e)),
-                       dmul(dmul(0.5, ro3), dadd(dadd(dmul(u3, u3), dmul(v3, v3)), 0.0))),
-                  gm1);
-    }
+    const double i3 = rs_rcp(ro3);
+    const double u3 = mx * i3;
+    double v3 = my * i3;
+    double p3 = fma(-0.5 * ro3, fma(v3, v3, u3 * u3), e3) * kG1;
     int rc = 0;
     if (p3 <= 0.0) {
         p3 = kPFloor;
         rc = 2;
     }
     if (x > (double)0.28f && y < (double)0.07f && v3 < 0.0) v3 = (double)0.01f;
-    const double qn[8] = {ro3, u3, v3, 0.0, p3, 0.0, 0.0, 0.0};
-    cons_from_prim_exact(qn, un);
+    un[0] = ro3;
+    un[1] = ro3 * u3;
+    un[2] = ro3 * v3;
+    un[4] = fma(0.5 * ro3, fma(v3, v3, u3 * u3), kInvG1 * p3);
+    un[3] = un[5] = un[6] = un[7] = 0.0;
     return rc;
 }
 
-// One face per thread, cuf_solvers.cuf:243-440 (face speed 0).
-template <int NSTATE, int ORDER, bool WANT_DT>
-__global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FaceListDev m, double cfl, int n_disc,
+// One face per thread, cuf_solvers.cuf:243-440 (face speed 0).  Bound by the latency of its gathers
+// and of dependent FP64 operations at 16 warps per SM (128 registers, no spills).  A face's four
+// cells are one 16-byte index load; the solver is the Cartesian path's (riemann_fp64.cuh) on any
+// tangents.  With the cell kernel below, a stage on a 96x80x64 box took 0.235 / 0.225 ms with the
+// library-division solver on the reference's field-aligned basis, a primitive pass before every
+// stage and three index arrays, and 0.169 / 0.167 ms so.
+// The distance-weighted face value of cell 1, linear(-dff1, q11, -df1, q1, df2, q2) at 0
+// (Solvers.f90:141-150), is q1 + minmod((q1 - q11) df1/(dff1 - df1), (q2 - q1) df1/(df1 + df2)): the
+// weights are geometry, formed at set-up (geo = df1, df1/(df1 + df2), df1/(dff1 - df1),
+// df2/(dff2 - df2); the second weight of side 2 is one minus that of side 1).
+// FAST: n_disc is 0 (HLLC / HLLD by the FP64 solvers).  LAX: the grid may have Lax faces (physics 1).
+template <int NSTATE, int ORDER, bool WANT_DT, bool FAST, bool LAX>
+__global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m, double cfl, int n_disc,
                                                                DevClock* clk, DevStatus* st) {
     __shared__ double red[kFaceThreads / 32];
     __shared__ unsigned long long cnt[2];
@@ -223,54 +240,45 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FaceList
     const int tword = gr < m.n_gran ? m.type[gr] : 0;
     const int type = tword & 7;
     if (type != 0) {
-        const int64_t s1 = m.nb[2 * gr] - 1;
-        const int32_t s2r = m.nb[2 * gr + 1];
-        const double n[3] = {m.normal[3 * gr], m.normal[3 * gr + 1], m.normal[3 * gr + 2]};
+        const int4 nb = __ldg(reinterpret_cast<const int4*>(m.nb) + gr);
+        const double2* n2 = reinterpret_cast<const double2*>(m.normal + 4 * gr);
+        const double2 na = __ldg(n2);
+        const double n[3] = {na.x, na.y, __ldg(m.normal + 4 * gr + 2)};
+        const double2* g2 = reinterpret_cast<const double2*>(m.geo + 4 * gr);
+        const double2 ga = __ldg(g2);
         double q1[8], q2[8];
-        load_prim(m.prim, s1, q1);
-        bool tvd = ORDER == 2;
+        load_prim(m.prim, nb.x, q1);
+        load_prim(m.prim, nb.y, q2);              // a ghost face: cell 1 again
         if (type == 4) {                          // :318-324 outer boundary
-#pragma unroll
-            for (int v = 0; v < 8; v++) q2[v] = q1[v];
             if (q2[1] > -0.1) q2[1] = -0.1;
-            tvd = false;
         } else if (type == 5) {                   // :325-329 axis
-#pragma unroll
-            for (int v = 0; v < 8; v++) q2[v] = q1[v];
             q2[2] = -q2[2];
-            tvd = false;
-        } else if (type == 2 && s2r == -1) {      // :330-345 reflecting wall
+        } else if (type == 2) {                   // :330-345 reflecting wall
             const double vel = dadd(dadd(dmul(n[0], q1[1]), dmul(n[1], q1[2])), dmul(n[2], q1[3]));
 #pragma unroll
-            for (int v = 0; v < 8; v++) q2[v] = q1[v];
-#pragma unroll
             for (int a = 0; a < 3; a++) q2[1 + a] = dsub(dsub(q1[1 + a], dmul(vel, n[a])), dmul(vel, n[a]));
-            tvd = false;
-        } else {
-            load_prim(m.prim, (int64_t)s2r - 1, q2);
-        }
-        const int32_t ss1 = m.nbt[2 * gr], ss2 = m.nbt[2 * gr + 1];
-        const double dist = m.geo[4 * gr];
-        if (tvd && ss1 >= 1 && ss2 >= 1) {       // :358-412, linear on the precomputed distances
-            const double df1 = dist, df2 = m.geo[4 * gr + 1], dff1 = m.geo[4 * gr + 2], dff2 = m.geo[4 * gr + 3];
-            double q11[8], q22[8];
-            load_prim(m.prim, (int64_t)ss1 - 1, q11);
-            load_prim(m.prim, (int64_t)ss2 - 1, q22);
+        } else if (ORDER == 2 && nb.z >= 0) {     // :358-412
+            const double2 gb = __ldg(g2 + 1);
+            double q11[6], q22[6];
+            load_prim<6>(m.prim, nb.z, q11);
+            load_prim<6>(m.prim, nb.w, q22);
+            const double b1 = ga.y, b2 = 1.0 - ga.y;
             double t1[5], t2[5];
 #pragma unroll
-            // linear(-dff1, q11, -df1, q1, df2, q2) and linear(-dff2, q22, -df2, q2, df1, q1): three
-            // reciprocals per face instead of 20 divisions (the face-list path measured 7 % faster)
-            const double ra1 = sb_rcp(dsub(-dff1, -df1)), ra2 = sb_rcp(dsub(-dff2, -df2));
-            const double rb = sb_rcp(dsub(-df1, df2));   // (-df2) - df1 rounds to the same value
-#pragma unroll
             for (int v = 0; v < 5; v++) {
-                t1[v] = linear_rcp(ra1, q11[v], -df1, q1[v], rb, q2[v]);
-                t2[v] = linear_rcp(ra2, q22[v], -df2, q2[v], rb, q1[v]);
+                const double dq = q2[v] - q1[v];
+                double h;
+                const double m1 = slope((q1[v] - q11[v]) * gb.x, dq * b1, h);
+                t1[v] = fma(h + h, m1, q1[v]);
+                const double m2 = slope(dq * b2, (q22[v] - q2[v]) * gb.y, h);
+                t2[v] = fma(-(h + h), m2, q2[v]);
             }
-            if (sb_neg(t1[0])) t1[0] = q1[0];
-            if (sb_neg(t1[4])) t1[4] = q1[4];
-            if (sb_neg(t2[0])) t2[0] = q2[0];
-            if (sb_neg(t2[4])) t2[4] = q2[4];
+            if (sb_neg(sum_neg(t1[0], t1[4], t2[0], t2[4]))) {
+                if (sb_neg(t1[0])) t1[0] = q1[0];
+                if (sb_neg(t1[4])) t1[4] = q1[4];
+                if (sb_neg(t2[0])) t2[0] = q2[0];
+                if (sb_neg(t2[4])) t2[4] = q2[4];
+            }
 #pragma unroll
             for (int v = 0; v < 5; v++) {
                 q1[v] = t1[v];
@@ -278,33 +286,37 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FaceList
             }
         }
         if (sb_neg(q1[0]) || sb_neg(q2[0])) n_recon++;
-        double qqq[8], sp[3];
-        int32_t fl = 0;
+        if (m.powell) {   // :433 as commented there: 0.5 * n.(B1 + B2) * square, B of the chlld states
+            const double nbs = dadd(dadd(dmul(n[0], dadd(q1[5], q2[5])), dmul(n[1], dadd(q1[6], q2[6]))),
+                                    dmul(n[2], dadd(q1[7], q2[7])));
+            m.divb[gr] = dmul(dmul(0.5 * kSpi4, nbs), __ldg(m.normal + 4 * gr + 3));
+        }
+        double F[8], SL, SR;
+        bool none;
+        auto reload = [&](double* m3) {
+            asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(m3[0]), "=d"(m3[1]) : "l"(n2));
+            asm volatile("ld.global.f64 %0, [%1];" : "=d"(m3[2]) : "l"(n2 + 1));
+        };
         // the faces do not move (w = 0): no face-speed terms
-        if (tword & kLaxFace) chlld_general<double, 0, false, false>(n, 0.0, q1, q2, n_disc, qqq, sp, &fl);   // :293-295
-        else chlld_general<double, NSTATE, false, false>(n, 0.0, q1, q2, n_disc, qqq, sp, &fl);
-        if (fl & kFlagWave) {
+        if (LAX && (tword & kLaxFace)) none = flux_normal_fp64<0, false>(n, reload, q1, q2, n_disc, F, SL, SR);   // :293-295
+        else none = flux_normal_fp64<NSTATE, FAST>(n, reload, q1, q2, n_disc, F, SL, SR);
+        if (none) {
             n_wave++;
 #pragma unroll
-            for (int v = 0; v < 8; v++) qqq[v] = 0.0;
+            for (int v = 0; v < 8; v++) F[v] = 0.0;
         }
-        const double sq = m.square[gr];
+        const double sq = __ldg(m.normal + 4 * gr + 3);
         double2* f2 = reinterpret_cast<double2*>(m.flux + 8 * gr);
 #pragma unroll
-        for (int v = 0; v < 4; v++) f2[v] = make_double2(qqq[2 * v] * sq, qqq[2 * v + 1] * sq);
-        if (m.powell) {   // :433 as commented there: 0.5 * n.(B1 + B2) * square, B of the chlld states
-            const double nb = dadd(dadd(dmul(n[0], dadd(q1[5], q2[5])), dmul(n[1], dadd(q1[6], q2[6]))),
-                                   dmul(n[2], dadd(q1[7], q2[7])));
-            m.divb[gr] = dmul(dmul(0.5, nb), sq);
-        }
+        for (int v = 0; v < 4; v++) f2[v] = make_double2(F[2 * v] * sq, F[2 * v + 1] * sq);
         // compare-and-select min / max (the library fmin / fmax of doubles are far longer sequences)
-        if (WANT_DT) cand = sb_min(kDtFaceCap, cfl * dist * sb_rcp(sb_max(fabs(sp[0]), fabs(sp[1]))));
+        if (WANT_DT) cand = sb_min(kDtFaceCap, cfl * ga.x * rs_rcp(sb_max(fabs(SL), fabs(SR))));
     }
     if (n_recon) atomicAdd(&cnt[0], (unsigned long long)n_recon);
     if (n_wave) atomicAdd(&cnt[1], (unsigned long long)n_wave);
     if (WANT_DT) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cand = fmin(cand, __shfl_xor_sync(0xffffffffu, cand, o));
+        for (int o = 16; o > 0; o >>= 1) cand = sb_min(cand, __shfl_xor_sync(0xffffffffu, cand, o));
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cand;
     }
     __syncthreads();
@@ -312,7 +324,7 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FaceList
         if (WANT_DT) {
             double r = red[0];
 #pragma unroll
-            for (int w = 1; w < kFaceThreads / 32; w++) r = fmin(r, red[w]);
+            for (int w = 1; w < kFaceThreads / 32; w++) r = sb_min(r, red[w]);
             atomicMin(&clk->dt_next, (unsigned long long)__double_as_longlong(r));
         }
         if (cnt[0]) atomicAdd(&st->n_recon, cnt[0]);
@@ -320,17 +332,59 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FaceList
     }
 }
 
-// One cell per thread, cuf_solvers.cuf:561-794 as the conservative MHD update: owner-signed sum
-// of the face fluxes (:691-703), Euler / Heun stage (:705-770), negative-density check, p floor
-// (:777-779), frozen cells (:611) and the re-imposed source sphere.  The last block of a
-// finalizing launch rolls the clock.
+// Owner-signed sum of a cell's face fluxes (:691-703), in the order of its face list.  All gathers of
+// three faces are in flight together; a missing face reads the zero row.
+template <bool POWELL>
+__device__ __forceinline__ void sum_fluxes(const FlView& m, int64_t c, double* pot, double& sks) {
+    const int2* j2 = reinterpret_cast<const int2*>(m.cell_gran + 6 * c);
+    int j[6];
+#pragma unroll
+    for (int f = 0; f < 3; f++) {
+        const int2 p = __ldg(j2 + f);
+        j[2 * f] = p.x;
+        j[2 * f + 1] = p.y;
+    }
+    sks = 0.0;
+#pragma unroll
+    for (int v = 0; v < 8; v++) pot[v] = 0.0;
+#pragma unroll
+    for (int g = 0; g < 6; g += 3) {
+        double2 d[3][4];
+        double db[3];
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            const int a = abs(j[g + f]);
+            const int64_t row = a ? a - 1 : m.n_gran;
+            const double2* f2 = reinterpret_cast<const double2*>(m.flux + 8 * row);
+#pragma unroll
+            for (int v = 0; v < 4; v++) d[f][v] = f2[v];
+            if (POWELL) db[f] = m.divb[row];
+        }
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            const double s = j[g + f] < 0 ? -1.0 : 1.0;
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                pot[2 * v] = fma(s, d[f][v].x, pot[2 * v]);
+                pot[2 * v + 1] = fma(s, d[f][v].y, pot[2 * v + 1]);
+            }
+            if (POWELL) sks = fma(s, db[f], sks);
+        }
+    }
+}
+
+// One cell per thread, cuf_solvers.cuf:561-794 as the conservative MHD update: flux sum, Euler / Heun
+// stage (:705-770), negative-density check, p floor (:777-779), frozen cells (:611) and the re-imposed
+// source sphere.  The new state's primitives go to m.prim where a next stage of the call reads them
+// (`more`), so no pass of its own re-reads the state.  The last block of a finalizing launch rolls the
+// clock.
 // PHYS: the physics option; POWELL: the div-B terms are on (their energy term by m.powell ==
 // 2).  Compile-time, so a launch carries only its own code (registers set the occupancy of this
 // gather-bound kernel).
 template <int KIND, int PHYS, bool POWELL>
-__global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FaceListDev m, const double* __restrict__ Uin,
+__global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, const double* __restrict__ Uin,
                                                                const double* Ubase, double* Uout, int64_t vs,
-                                                               DevClock* clk, DevStatus* st, int finalize) {
+                                                               DevClock* clk, DevStatus* st, int finalize, int more) {
     __shared__ unsigned long long cnt[2];
     __shared__ bool last;
     if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
@@ -338,33 +392,22 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FaceListDev
     const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const double dt = clk->dt_cur;
     if (c < m.n_cell) {
-        double un[8], qs[8];
-        const double x = m.cell_center[3 * c], y = m.cell_center[3 * c + 1], z = m.cell_center[3 * c + 2];
-        const double r2 = dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z));
-        if (m.cell_flag[c] & 1) {
+        double un[8], q[8];
+        bool have_q = false;
+        const int flag = m.cell_flag[c];
+        if (flag & kFrozen) {
 #pragma unroll
             for (int v = 0; v < 8; v++) un[v] = KIND == 0 ? Uin[v * vs + c] : Ubase[v * vs + c];
-        } else if (PHYS == 0 && m.src.r_src > 0.0 && r2 < dmul(m.src.r_src, m.src.r_src)) {
-            source_state(m.src, x, y, z, r2, qs);
-            cons_from_prim_exact(qs, un);
+        } else if (PHYS == 0 && (flag & kSource)) {
+            const double x = m.cell_center[3 * c], y = m.cell_center[3 * c + 1], z = m.cell_center[3 * c + 2];
+            source_state(m.src, x, y, z, dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z)), q);
+            cons_from_prim_exact(q, un);
         } else if (PHYS == 1) {
-            double pot[8];
-#pragma unroll
-            for (int v = 0; v < 8; v++) pot[v] = 0.0;
-            for (int f = 0; f < 6; f++) {
-                const int32_t j = m.cell_gran[6 * c + f];
-                if (j == 0) continue;
-                const int64_t jf = (int64_t)j - 1;
-                const bool owner = m.nb[2 * jf] == (int32_t)(c + 1);
-                const double2* f2 = reinterpret_cast<const double2*>(m.flux + 8 * jf);
-#pragma unroll
-                for (int v = 0; v < 4; v++) {
-                    const double2 d = f2[v];
-                    pot[2 * v] = owner ? pot[2 * v] + d.x : pot[2 * v] - d.x;
-                    pot[2 * v + 1] = owner ? pot[2 * v + 1] + d.y : pot[2 * v + 1] - d.y;
-                }
-            }
-            const int rc = axisym_update<KIND>(Uin, Ubase, vs, c, pot, m.cell_volume[c], x, y, m.hatom + 8 * c, dt, un);
+            double pot[8], sks;
+            sum_fluxes<false>(m, c, pot, sks);
+            load_prim(m.prim, c, q);
+            const int rc = axisym_update<KIND>(Uin, Ubase, vs, c, q, pot, m.inv_volume[c], m.cell_center[3 * c],
+                                               m.cell_center[3 * c + 1], m.hatom + 8 * c, dt, un);
             if (rc == 1) {
                 atomicAdd(&cnt[0], 1ull);
                 atomicMin(&st->first_bad, (unsigned long long)c);
@@ -372,48 +415,34 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FaceListDev
                 atomicAdd(&cnt[1], 1ull);
             }
         } else {
-            double pot[8], sks = 0.0;
-#pragma unroll
-            for (int v = 0; v < 8; v++) pot[v] = 0.0;
-            for (int f = 0; f < 6; f++) {
-                const int32_t j = m.cell_gran[6 * c + f];
-                if (j == 0) continue;
-                const int64_t jf = (int64_t)j - 1;
-                const bool owner = m.nb[2 * jf] == (int32_t)(c + 1);
-                const double2* f2 = reinterpret_cast<const double2*>(m.flux + 8 * jf);
-#pragma unroll
-                for (int v = 0; v < 4; v++) {
-                    const double2 d = f2[v];
-                    pot[2 * v] = owner ? pot[2 * v] + d.x : pot[2 * v] - d.x;
-                    pot[2 * v + 1] = owner ? pot[2 * v + 1] + d.y : pot[2 * v + 1] - d.y;
-                }
-                if (POWELL) sks = owner ? sks + m.divb[jf] : sks - m.divb[jf];
-            }
+            double pot[8], sks;
+            sum_fluxes<POWELL>(m, c, pot, sks);
             if (POWELL) {
                 // div-B sources inside the flux sum (cuf_solvers.cuf:529-533 / 729-733, commented
                 // there): momentum + (B/4pi) sks, B + u sks, powell 2 energy + (u.B/4pi) sks, with
-                // u and B of the stage input (the primitive pass of this stage)
-                double q[8];
+                // u and B of the stage input (its primitive state); b = B / sqrt(4 pi), and the field
+                // sums are in units of b
                 load_prim(m.prim, c, q);
+                const double sb = sks * kInvSpi4;
 #pragma unroll
                 for (int a = 0; a < 3; a++) {
-                    pot[1 + a] = dadd(pot[1 + a], dmul(q[5 + a] / kCpi4, sks));
-                    pot[5 + a] = dadd(pot[5 + a], dmul(q[1 + a], sks));
+                    pot[1 + a] = dadd(pot[1 + a], dmul(q[5 + a], sb));
+                    pot[5 + a] = dadd(pot[5 + a], dmul(q[1 + a], sb));
                 }
                 if (m.powell == 2) {
                     const double ub = dadd(dadd(dmul(q[1], q[5]), dmul(q[2], q[6])), dmul(q[3], q[7]));
-                    pot[4] = dadd(pot[4], dmul(ub / kCpi4, sks));
+                    pot[4] = dadd(pot[4], dmul(ub, sb));
                 }
             }
-            // one reciprocal of the volume instead of eight divisions (the face-list path measured
-            // 7 % faster); the dt candidate below likewise multiplies by 1/max(|SL|,|SR|)
-            const double ivol = sb_rcp(m.cell_volume[c]);
+            const double ivol = m.inv_volume[c];
+            const double ivb = ivol * kSpi4;   // field fluxes are in units of b
             double uin[8];
 #pragma unroll
             for (int v = 0; v < 8; v++) {
                 uin[v] = Uin[v * vs + c];
-                if (KIND == 0) un[v] = uin[v] - dt * (pot[v] * ivol);
-                else un[v] = 0.5 * ((Ubase[v * vs + c] + uin[v]) - dt * (pot[v] * ivol));
+                const double d = pot[v] * (v < 5 ? ivol : ivb);
+                if (KIND == 0) un[v] = uin[v] - dt * d;
+                else un[v] = 0.5 * ((Ubase[v * vs + c] + uin[v]) - dt * d);
             }
             if (!(un[0] > 0.0)) {
                 atomicAdd(&cnt[0], 1ull);
@@ -421,16 +450,25 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FaceListDev
 #pragma unroll
                 for (int v = 0; v < 8; v++) un[v] = uin[v];
             } else {
-                double q[8], ke, me;
-                prim_from_cons(un, q, ke, me);
+                double ke, me;
+                prim_from_cons<true, true>(un, q, ke, me);
+                have_q = true;
                 if (q[4] <= 0.0) {
                     atomicAdd(&cnt[1], 1ull);
                     un[4] = floor_energy(ke, me);
+                    have_q = false;
                 }
             }
         }
 #pragma unroll
         for (int v = 0; v < 8; v++) Uout[v * vs + c] = un[v];
+        if (more) {
+            if (!have_q) {
+                double ke, me;
+                prim_from_cons<true, true>(un, q, ke, me);
+            }
+            store_prim(m.prim, c, q);
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -454,16 +492,29 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FaceListDev
     }
 }
 
-template <int NSTATE>
-void launch_face_n(const FaceListDev& m, int order, bool want_dt, double cfl, int n_disc, DevClock* clk,
-                   DevStatus* st, cudaStream_t s) {
+template <int NSTATE, int ORDER, bool WANT_DT>
+void launch_face_o(const FlView& m, bool lax, double cfl, int n_disc, DevClock* clk, DevStatus* st, cudaStream_t s) {
+    constexpr bool HAS_FAST = NSTATE >= 2;
     const unsigned grid = (unsigned)((m.n_gran + kFaceThreads - 1) / kFaceThreads);
-    if (order == 2) {
-        if (want_dt) fl_face_kernel<NSTATE, 2, true><<<grid, kFaceThreads, 0, s>>>(m, cfl, n_disc, clk, st);
-        else fl_face_kernel<NSTATE, 2, false><<<grid, kFaceThreads, 0, s>>>(m, cfl, n_disc, clk, st);
+#define SB_FACE(F, L) fl_face_kernel<NSTATE, ORDER, WANT_DT, F, L><<<grid, kFaceThreads, 0, s>>>(m, cfl, n_disc, clk, st)
+    if (HAS_FAST && n_disc == 0) {
+        if (lax) SB_FACE(HAS_FAST, true);
+        else SB_FACE(HAS_FAST, false);
     } else {
-        if (want_dt) fl_face_kernel<NSTATE, 1, true><<<grid, kFaceThreads, 0, s>>>(m, cfl, n_disc, clk, st);
-        else fl_face_kernel<NSTATE, 1, false><<<grid, kFaceThreads, 0, s>>>(m, cfl, n_disc, clk, st);
+        SB_FACE(false, true);
+    }
+#undef SB_FACE
+}
+
+template <int NSTATE>
+void launch_face_n(const FlView& m, bool lax, int order, bool want_dt, double cfl, int n_disc, DevClock* clk,
+                   DevStatus* st, cudaStream_t s) {
+    if (order == 2) {
+        if (want_dt) launch_face_o<NSTATE, 2, true>(m, lax, cfl, n_disc, clk, st, s);
+        else launch_face_o<NSTATE, 2, false>(m, lax, cfl, n_disc, clk, st, s);
+    } else {
+        if (want_dt) launch_face_o<NSTATE, 1, true>(m, lax, cfl, n_disc, clk, st, s);
+        else launch_face_o<NSTATE, 1, false>(m, lax, cfl, n_disc, clk, st, s);
     }
 }
 
@@ -472,9 +523,9 @@ void launch_face_n(const FaceListDev& m, int order, bool want_dt, double cfl, in
 // ------------------------------------------------------------------------------ host side
 void fl_destroy(FaceListDev* f) {
     if (!f) return;
-    void* ptrs[] = {f->cell_center, f->cell_volume, f->cell_gran, f->cell_flag, f->normal, f->square, f->geo,
-                    f->nb,          f->nbt,         f->type,      f->prim,      f->flux,   f->hatom,
-                    f->divb};
+    const FlView& m = f->v;
+    void* ptrs[] = {m.cell_center, m.inv_volume, m.cell_gran, m.cell_flag, m.normal, m.geo, m.nb,
+                    m.type,        m.prim,       m.flux,      m.hatom,     m.divb};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete f;
@@ -560,98 +611,90 @@ int fl_create(FaceListDev** out, int64_t N, int64_t G, const double* cell_center
         });
         for (int64_t d = 0; d < G; d++) fnew[fperm[d]] = (int32_t)d;
     }
-    auto cell_ref = [&](int32_t c1) { return c1 >= 1 ? cnew[c1 - 1] + 1 : c1; };   // 1-based, -1 kept
-    std::vector<double> cell_center((size_t)N * 3), cell_volume((size_t)N), gran_normal((size_t)G * 3),
-        gran_square((size_t)G), gran_center((size_t)G * 3);
-    std::vector<int32_t> cell_gran((size_t)N * 6), gran_neighbour((size_t)G * 2), gran_neighbour_tvd((size_t)G * 2),
-        gran_type_v((size_t)G);
-    for (int64_t d = 0; d < N; d++) {
-        const int64_t c = cperm[d];
-        for (int a = 0; a < 3; a++) cell_center[3 * d + a] = cell_center_in[3 * c + a];
-        cell_volume[d] = cell_volume_in[c];
-        for (int f = 0; f < 6; f++) {
-            const int32_t j = cell_gran_in[6 * c + f];
-            cell_gran[6 * d + f] = j >= 1 ? fnew[j - 1] + 1 : 0;
-        }
-    }
+    auto cell_ref = [&](int32_t c1) { return cnew[c1 - 1]; };   // caller's 1-based -> device 0-based
+    std::vector<double> cell_center((size_t)N * 3), inv_volume((size_t)N), geo((size_t)G * 4), normal4((size_t)G * 4);
+    std::vector<int32_t> cell_gran((size_t)N * 6), type((size_t)G), nb((size_t)G * 4);
     for (int64_t d = 0; d < G; d++) {
         const int64_t g = fperm[d];
-        for (int a = 0; a < 3; a++) {
-            gran_normal[3 * d + a] = gran_normal_in[3 * g + a];
-            gran_center[3 * d + a] = gran_center_in[3 * g + a];
-        }
-        gran_square[d] = gran_square_in[g];
-        for (int b = 0; b < 2; b++) {
-            gran_neighbour[2 * d + b] = cell_ref(gran_neighbour_in[2 * g + b]);
-            gran_neighbour_tvd[2 * d + b] = cell_ref(gran_neighbour_tvd_in[2 * g + b]);
-        }
-        gran_type_v[d] = gran_type_in[g];
-    }
-    const int32_t* gran_type = gran_type_v.data();
-    std::vector<double> geo((size_t)G * 4);
-    std::vector<int32_t> type((size_t)G);
-    for (int64_t g = 0; g < G; g++) {
-        const int32_t s1 = gran_neighbour[2 * g], s2 = gran_neighbour[2 * g + 1];
-        const int32_t t = gran_type[g];
-        const int32_t ss1 = gran_neighbour_tvd[2 * g], ss2 = gran_neighbour_tvd[2 * g + 1];
+        const int32_t s1 = gran_neighbour_in[2 * g], s2 = gran_neighbour_in[2 * g + 1], t = gran_type_in[g];
+        const int32_t ss1 = gran_neighbour_tvd_in[2 * g], ss2 = gran_neighbour_tvd_in[2 * g + 1];
         const bool ghost = t == 4 || t == 5 || (t == 2 && s2 == -1);
         // distances as the reference forms them each step (cuf_solvers.cuf:290-292, 362-372)
-        const double* gc = gran_center.data() + 3 * g;
-        const double* c1 = cell_center.data() + 3 * (int64_t)(s1 - 1);
-        const double* c2 = ghost ? c1 : cell_center.data() + 3 * (int64_t)(s2 - 1);
-        double r[3];
-        for (int a = 0; a < 3; a++) r[a] = gc[a] - c1[a];
-        geo[4 * g] = norm3(r);
-        for (int a = 0; a < 3; a++) r[a] = gc[a] - c2[a];
-        geo[4 * g + 1] = norm3(r);
-        geo[4 * g + 2] = geo[4 * g + 3] = 0.0;
-        if (ss1 >= 1) {
-            for (int a = 0; a < 3; a++) r[a] = gc[a] - cell_center[3 * (int64_t)(ss1 - 1) + a];
-            geo[4 * g + 2] = norm3(r);
+        const double* gc = gran_center_in + 3 * g;
+        auto distance = [&](int32_t c) {
+            const double* x = cell_center_in + 3 * (int64_t)(c - 1);
+            const double r[3] = {gc[0] - x[0], gc[1] - x[1], gc[2] - x[2]};
+            return norm3(r);
+        };
+        const double df1 = distance(s1);
+        geo[4 * d] = df1;
+        const bool tvd = !ghost && ss1 >= 1 && ss2 >= 1;
+        if (tvd) {
+            const double df2 = distance(s2), dff1 = distance(ss1), dff2 = distance(ss2);
+            geo[4 * d + 1] = df1 / (df1 + df2);
+            geo[4 * d + 2] = df1 / (dff1 - df1);
+            geo[4 * d + 3] = df2 / (dff2 - df2);
         }
-        if (ss2 >= 1) {
-            for (int a = 0; a < 3; a++) r[a] = gc[a] - cell_center[3 * (int64_t)(ss2 - 1) + a];
-            geo[4 * g + 3] = norm3(r);
-        }
+        const double* n = gran_normal_in + 3 * g;
+        for (int a = 0; a < 3; a++) normal4[4 * d + a] = n[a];
+        normal4[4 * d + 3] = gran_square_in[g];
+        nb[4 * d] = cell_ref(s1);
+        nb[4 * d + 1] = ghost ? nb[4 * d] : cell_ref(s2);
+        nb[4 * d + 2] = tvd ? cell_ref(ss1) : -1;
+        nb[4 * d + 3] = tvd ? cell_ref(ss2) : -1;
         // the reference skips faces whose first cell lies inside its frozen core (:284)
-        type[g] = (p->face_skip_radius > 0.0 && norm3(c1) < p->face_skip_radius) ? 0 : t;
+        const double* c1 = cell_center_in + 3 * (int64_t)(s1 - 1);
+        type[d] = (p->face_skip_radius > 0.0 && norm3(c1) < p->face_skip_radius) ? 0 : (t == 2 && !ghost ? kInner : t);
         // physics 1: the reference's Lax flux on faces near the axis (cuf_solvers.cuf:293-295)
-        if (type[g] && p->physics == 1 && gc[0] > (double)0.22f && gc[1] < (double)0.1f &&
-            std::fabs(gran_normal[3 * g]) < (double)0.1f)
-            type[g] |= kLaxFace;
+        if (type[d] && p->physics == 1 && gc[0] > (double)0.22f && gc[1] < (double)0.1f &&
+            std::fabs(n[0]) < (double)0.1f)
+            type[d] |= kLaxFace;
     }
     std::vector<unsigned char> flag((size_t)N);
-    for (int64_t c = 0; c < N; c++)
-        flag[c] = (p->cell_freeze_radius > 0.0 && norm3(cell_center.data() + 3 * c) < p->cell_freeze_radius) ? 1 : 0;
+    for (int64_t d = 0; d < N; d++) {
+        const int64_t c = cperm[d];
+        const double* x = cell_center_in + 3 * c;
+        for (int a = 0; a < 3; a++) cell_center[3 * d + a] = x[a];
+        const double r2 = (x[0] * x[0] + x[1] * x[1]) + x[2] * x[2];
+        flag[d] = ((p->cell_freeze_radius > 0.0 && norm3(x) < p->cell_freeze_radius) ? kFrozen : 0) |
+                  ((p->r_src > 0.0 && r2 < p->r_src * p->r_src) ? kSource : 0);
+        inv_volume[d] = 1.0 / cell_volume_in[c];
+        for (int f = 0; f < 6; f++) {   // the face, positive where this cell is its first neighbour
+            const int32_t j = cell_gran_in[6 * c + f];
+            if (j < 1) continue;
+            const int32_t jd = fnew[j - 1] + 1;
+            cell_gran[6 * d + f] = gran_neighbour_in[2 * (int64_t)(j - 1)] == (int32_t)(c + 1) ? jd : -jd;
+        }
+    }
 
     FaceListDev* f = new (std::nothrow) FaceListDev();
     if (!f) return SETB_ENOMEM;
-    f->n_cell = N;
-    f->n_gran = G;
-    f->src.r_src = p->r_src;
-    f->src.rho_src = p->rho_src;
-    f->src.v_src = p->v_src;
-    f->src.p_over_rho_src = p->p_over_rho_src;
-    f->src.r_floor = p->r_floor;
+    FlView& m = f->v;
+    m.n_cell = N;
+    m.n_gran = G;
+    m.src.r_src = p->r_src;
+    m.src.rho_src = p->rho_src;
+    m.src.v_src = p->v_src;
+    m.src.p_over_rho_src = p->p_over_rho_src;
+    m.src.r_floor = p->r_floor;
+    m.powell = p->powell;
     f->perm = cperm;
     f->physics = p->physics;
-    f->powell = p->powell;
-    bool ok = upload(&f->cell_center, cell_center.data(), 3 * (size_t)N, s) == cudaSuccess &&
-              upload(&f->cell_volume, cell_volume.data(), (size_t)N, s) == cudaSuccess &&
-              upload(&f->cell_gran, cell_gran.data(), 6 * (size_t)N, s) == cudaSuccess &&
-              upload(&f->cell_flag, flag.data(), (size_t)N, s) == cudaSuccess &&
-              upload(&f->normal, gran_normal.data(), 3 * (size_t)G, s) == cudaSuccess &&
-              upload(&f->square, gran_square.data(), (size_t)G, s) == cudaSuccess &&
-              upload(&f->geo, geo.data(), 4 * (size_t)G, s) == cudaSuccess &&
-              upload(&f->nb, gran_neighbour.data(), 2 * (size_t)G, s) == cudaSuccess &&
-              upload(&f->nbt, gran_neighbour_tvd.data(), 2 * (size_t)G, s) == cudaSuccess &&
-              upload(&f->type, type.data(), (size_t)G, s) == cudaSuccess &&
-              cudaMalloc(&f->prim, sizeof(double) * 8 * (size_t)N) == cudaSuccess &&
-              cudaMalloc(&f->flux, sizeof(double) * 8 * (size_t)G) == cudaSuccess &&
-              (p->physics != 1 || cudaMalloc(&f->hatom, sizeof(double) * 8 * (size_t)N) == cudaSuccess) &&
-              cudaMemsetAsync(f->flux, 0, sizeof(double) * 8 * (size_t)G, s) == cudaSuccess &&
-              (p->powell == 0 || (cudaMalloc(&f->divb, sizeof(double) * (size_t)G) == cudaSuccess &&
-                                  cudaMemsetAsync(f->divb, 0, sizeof(double) * (size_t)G, s) == cudaSuccess)) &&
+    const size_t rows = (size_t)G + 1;
+    bool ok = upload(&m.cell_center, cell_center.data(), 3 * (size_t)N, s) == cudaSuccess &&
+              upload(&m.inv_volume, inv_volume.data(), (size_t)N, s) == cudaSuccess &&
+              upload(&m.cell_gran, cell_gran.data(), 6 * (size_t)N, s) == cudaSuccess &&
+              upload(&m.cell_flag, flag.data(), (size_t)N, s) == cudaSuccess &&
+              upload(&m.normal, normal4.data(), 4 * (size_t)G, s) == cudaSuccess &&
+              upload(&m.geo, geo.data(), 4 * (size_t)G, s) == cudaSuccess &&
+              upload(&m.nb, nb.data(), 4 * (size_t)G, s) == cudaSuccess &&
+              upload(&m.type, type.data(), (size_t)G, s) == cudaSuccess &&
+              cudaMalloc(&m.prim, sizeof(double) * 8 * (size_t)N) == cudaSuccess &&
+              cudaMalloc(&m.flux, sizeof(double) * 8 * rows) == cudaSuccess &&
+              (p->physics != 1 || cudaMalloc(&m.hatom, sizeof(double) * 8 * (size_t)N) == cudaSuccess) &&
+              cudaMemsetAsync(m.flux, 0, sizeof(double) * 8 * rows, s) == cudaSuccess &&
+              (p->powell == 0 || (cudaMalloc(&m.divb, sizeof(double) * rows) == cudaSuccess &&
+                                  cudaMemsetAsync(m.divb, 0, sizeof(double) * rows, s) == cudaSuccess)) &&
               cudaStreamSynchronize(s) == cudaSuccess;   // host vectors are released on return
     if (!ok) {
         cudaGetLastError();
@@ -664,19 +707,21 @@ int fl_create(FaceListDev** out, int64_t N, int64_t G, const double* cell_center
 
 cudaError_t fl_launch_stage(const FaceListDev* f, const double* Uin, const double* Ubase, double* Uout, int64_t vs,
                             DevClock* clk, DevStatus* st, const setb_step_opts* o, int kind, bool want_dt,
-                            bool finalize, cudaStream_t s) {
-    const FaceListDev& m = *f;
-    const unsigned pgrid = (unsigned)std::min<int64_t>((m.n_cell + kPrimThreads - 1) / kPrimThreads, 148 * 16);
-    fl_prim_kernel<<<pgrid, kPrimThreads, 0, s>>>(m.n_cell, Uin, vs, m.prim);
+                            bool finalize, bool first, bool more, cudaStream_t s) {
+    const FlView& m = f->v;
+    if (first) {
+        const unsigned pgrid = (unsigned)std::min<int64_t>((m.n_cell + kPrimThreads - 1) / kPrimThreads, 148 * 16);
+        fl_prim_kernel<<<pgrid, kPrimThreads, 0, s>>>(m.n_cell, Uin, vs, m.prim);
+    }
     switch (o->n_state) {
-        case 0: launch_face_n<0>(m, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
-        case 1: launch_face_n<1>(m, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
-        case 2: launch_face_n<2>(m, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
-        default: launch_face_n<3>(m, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
+        case 0: launch_face_n<0>(m, f->physics == 1, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
+        case 1: launch_face_n<1>(m, f->physics == 1, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
+        case 2: launch_face_n<2>(m, f->physics == 1, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
+        default: launch_face_n<3>(m, f->physics == 1, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
     }
     const unsigned cgrid = (unsigned)((m.n_cell + kCellThreads - 1) / kCellThreads);
-#define SB_CELL(K, PH, PW) fl_cell_kernel<K, PH, PW><<<cgrid, kCellThreads, 0, s>>>(m, Uin, Ubase, Uout, vs, clk, st, finalize)
-    if (m.physics == 1) {
+#define SB_CELL(K, PH, PW) fl_cell_kernel<K, PH, PW><<<cgrid, kCellThreads, 0, s>>>(m, Uin, Ubase, Uout, vs, clk, st, finalize, more)
+    if (f->physics == 1) {
         if (kind == 0) SB_CELL(0, 1, false);
         else SB_CELL(1, 1, false);
     } else if (m.powell) {
@@ -699,11 +744,11 @@ const int32_t* fl_perm(const FaceListDev* f) { return f ? f->perm.data() : nullp
 namespace sb {
 // Uploads the H-atom fluids (Cell_par columns 9..16, caller numbering) of a physics-1 face list.
 int fl_set_hatom(FaceListDev* f, const double* cell_par, cudaStream_t s) {
-    if (!f || !f->hatom) return SETB_OK;
-    const size_t N = (size_t)f->n_cell;
+    if (!f || !f->v.hatom) return SETB_OK;
+    const size_t N = (size_t)f->v.n_cell;
     std::vector<double> tmp(8 * N);
     for (size_t d = 0; d < N; d++) std::memcpy(&tmp[8 * d], cell_par + 16 * (size_t)f->perm[d] + 8, 8 * sizeof(double));
-    if (cudaMemcpyAsync(f->hatom, tmp.data(), sizeof(double) * 8 * N, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+    if (cudaMemcpyAsync(f->v.hatom, tmp.data(), sizeof(double) * 8 * N, cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return SETB_ECUDA;
     return SETB_OK;

@@ -192,39 +192,61 @@ __device__ __forceinline__ bool hlld_fp64(const double* q1, const double* q2, do
     return !(S2 <= 0.0) && !(S2 > 0.0) && !(SL > 0.0);
 }
 
-// HLLC with no magnetic field on either side (:1465-1567 with bn = 0): one sound speed a side, the
-// star state of the selected side alone; F[5..7] = 0.  Returns true when no region matched.
-__device__ __forceinline__ bool hllc_hydro_fp64(const double* q1, const double* q2, double* F, double& SLo,
-                                                double& SRo) {
-    const double r1 = q1[0], u1 = q1[1], p1 = q1[4], r2 = q2[0], u2 = q2[1], p2 = q2[4];
+// HLLC with no magnetic field on either side (:1465-1567 with bn = 0) from density, normal velocity and
+// pressure: one sound speed a side, the star state of the selected side alone.
+struct HydroFan {
+    double SL, SR, SM, ptz;
+    double r, u, p, su, rs, S;   // the selected side: state, S - u, rho (S - u), outer speed
+    bool right, none;            // none: no region matched
+    double F0, F1;               // mass and normal momentum flux
+};
+__device__ __forceinline__ void hllc_hydro_fan(double r1, double u1, double p1, double r2, double u2, double p2,
+                                               HydroFan& f) {
     // c = sqrt(gamma p / rho) = gamma p / sqrt(gamma p rho)
     const double g1 = fma(kGamma, p1, 1e-300), g2 = fma(kGamma, p2, 1e-300);
     const double c1 = over_sqrt(g1, g1 * r1), c2 = over_sqrt(g2, g2 * r2);
-    const double SL = sb_min(u1 - c1, u2 - c2), SR = sb_max(u1 + c1, u2 + c2);
-    SLo = SL;
-    SRo = SR;
-    const double su1 = SL - u1, su2 = SR - u2;
+    f.SL = sb_min(u1 - c1, u2 - c2);
+    f.SR = sb_max(u1 + c1, u2 + c2);
+    const double su1 = f.SL - u1, su2 = f.SR - u2;
     const double rs1 = r1 * su1, rs2 = r2 * su2;
-    const double SM = fma(rs2, u2, fma(-rs1, u1, p1 - p2)) * rs_rcp(rs2 - rs1);
-    const double ptz = 0.5 * (fma(rs2, SM - u2, p2) + fma(rs1, SM - u1, p1));
-    const bool right = !(SM > 0.0) || SR < 0.0;
-    const double r = pick(r1, r2, right), u = pick(u1, u2, right), p = pick(p1, p2, right);
-    const double v = pick(q1[2], q2[2], right), w = pick(q1[3], q2[3], right);
-    const double S = pick(SL, SR, right), su = pick(su1, su2, right), rs = pick(rs1, rs2, right);
-    const double Ss = (right ? SR >= 0.0 : SL <= 0.0) ? S : 0.0;   // 0 where the face lies outside the fan
-    const double i = rs_rcp(S - SM);
-    const double rz = rs * i;
-    const double m = r * u;
-    const double e = fma(0.5 * r, fma(w, w, fma(v, v, u * u)), 1.5 * p);
-    const double ez = fma(ptz, SM, fma(-p, u, e * su)) * i;
-    const double F0 = fma(Ss, rz - r, m);
-    F[0] = F0;
-    F[1] = fma(Ss, fma(rz, SM, -m), fma(m, u, p));
-    F[2] = F0 * v;   // m v + S (rho* - rho) v
-    F[3] = F0 * w;
-    F[4] = fma(Ss, ez - e, (e + p) * u);
+    f.SM = fma(rs2, u2, fma(-rs1, u1, p1 - p2)) * rs_rcp(rs2 - rs1);
+    f.ptz = 0.5 * (fma(rs2, f.SM - u2, p2) + fma(rs1, f.SM - u1, p1));
+    f.right = !(f.SM > 0.0) || f.SR < 0.0;
+    f.r = pick(r1, r2, f.right);
+    f.u = pick(u1, u2, f.right);
+    f.p = pick(p1, p2, f.right);
+    f.S = pick(f.SL, f.SR, f.right);
+    f.su = pick(su1, su2, f.right);
+    f.rs = pick(rs1, rs2, f.right);
+    f.none = !(f.SM <= 0.0) && !(f.SM > 0.0) && !(f.SL > 0.0) && !(f.SR < 0.0);
+}
+// Mass, normal momentum and energy flux; v2 = |v|^2 of the selected side.  The tangential momentum
+// flux is F0 times the selected side's tangential velocity (m v + S (rho* - rho) v).
+__device__ __forceinline__ double hllc_hydro_flux(HydroFan& f, double v2) {
+    const double Ss = (f.right ? f.SR >= 0.0 : f.SL <= 0.0) ? f.S : 0.0;   // 0 outside the fan
+    const double i = rs_rcp(f.S - f.SM);
+    const double rz = f.rs * i;
+    const double m = f.r * f.u;
+    const double e = fma(0.5 * f.r, v2, 1.5 * f.p);
+    const double ez = fma(f.ptz, f.SM, fma(-f.p, f.u, e * f.su)) * i;
+    f.F0 = fma(Ss, rz - f.r, m);
+    f.F1 = fma(Ss, fma(rz, f.SM, -m), fma(m, f.u, f.p));
+    return fma(Ss, ez - e, (e + f.p) * f.u);
+}
+__device__ __forceinline__ bool hllc_hydro_fp64(const double* q1, const double* q2, double* F, double& SLo,
+                                                double& SRo) {
+    HydroFan f;
+    hllc_hydro_fan(q1[0], q1[1], q1[4], q2[0], q2[1], q2[4], f);
+    SLo = f.SL;
+    SRo = f.SR;
+    const double v = pick(q1[2], q2[2], f.right), w = pick(q1[3], q2[3], f.right);
+    F[4] = hllc_hydro_flux(f, fma(w, w, fma(v, v, f.u * f.u)));
+    F[0] = f.F0;
+    F[1] = f.F1;
+    F[2] = f.F0 * v;
+    F[3] = f.F0 * w;
     F[5] = F[6] = F[7] = 0.0;
-    return !(SM <= 0.0) && !(SM > 0.0) && !(SL > 0.0) && !(SR < 0.0);
+    return f.none;
 }
 
 // Whether any of the six field components of the two states is nonzero.
@@ -251,6 +273,91 @@ __device__ __forceinline__ bool flux_fp64(const double* q1, const double* q2, do
         for (int v = 5; v < 8; v++) F[v] *= kInvSpi4;
         return (fl & kFlagWave) != 0;
     }
+}
+
+// Unit tangents (e2, e3) completing a unit normal to an orthonormal frame (T. Duff et al., "Building
+// an Orthonormal Basis, Revisited", JCGT 6(1), 2017).  The flux does not depend on which tangents are
+// taken: every formula treats the two tangential components as a 2-vector.
+__device__ __forceinline__ void tangent_frame(const double* n, double* e2, double* e3) {
+    const double s = copysign(1.0, n[2]);
+    const double a = -rs_rcp(s + n[2]);
+    const double b = n[0] * n[1] * a;
+    e2[0] = fma(s * n[0] * n[0], a, 1.0);
+    e2[1] = s * b;
+    e2[2] = -s * n[0];
+    e3[0] = b;
+    e3[1] = fma(n[1] * n[1], a, s);
+    e3[2] = -n[1];
+}
+__device__ __forceinline__ double dot3(const double* a, double x, double y, double z) {
+    return fma(a[2], z, fma(a[1], y, a[0] * x));
+}
+
+// The flux at a face of unit normal n (at rest) between lab states q (rho, u, v, w, p, b): F in lab
+// components, field fluxes in units of b.  NSTATE as riemann().  FAST: HLLC / HLLD for n_disc 0 by the
+// solvers above; otherwise riemann().
+// reload(m) gives the normal once more.
+template <int NSTATE, bool FAST, typename Reload>
+__device__ __forceinline__ bool flux_normal_fp64(const double* n, Reload reload, const double* q1, const double* q2,
+                                                 int n_disc, double* F, double& SL, double& SR) {
+    if constexpr (NSTATE == 2 && FAST) {
+        if (!__any_sync(__activemask(), has_field(q1, q2))) {
+            HydroFan f;
+            const double u1 = dot3(n, q1[1], q1[2], q1[3]), u2 = dot3(n, q2[1], q2[2], q2[3]);
+            hllc_hydro_fan(q1[0], u1, q1[4], q2[0], u2, q2[4], f);
+            SL = f.SL;
+            SR = f.SR;
+            double v[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) v[c] = pick(q1[1 + c], q2[1 + c], f.right);
+            F[4] = hllc_hydro_flux(f, fma(v[2], v[2], fma(v[1], v[1], v[0] * v[0])));
+            F[0] = f.F0;
+            const double fn = fma(-f.F0, f.u, f.F1);   // n F1 + F0 (v - u n)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                F[1 + c] = fma(fn, n[c], f.F0 * v[c]);
+                F[5 + c] = 0.0;
+            }
+            return f.none;
+        }
+    }
+    double e2[3], e3[3], a[8], b[8], G[8];
+    tangent_frame(n, e2, e3);
+    a[0] = q1[0];
+    a[4] = q1[4];
+    b[0] = q2[0];
+    b[4] = q2[4];
+#pragma unroll
+    for (int o = 1; o < 8; o += 4) {
+        a[o] = dot3(n, q1[o], q1[o + 1], q1[o + 2]);
+        a[o + 1] = dot3(e2, q1[o], q1[o + 1], q1[o + 2]);
+        a[o + 2] = dot3(e3, q1[o], q1[o + 1], q1[o + 2]);
+        b[o] = dot3(n, q2[o], q2[o + 1], q2[o + 2]);
+        b[o + 1] = dot3(e2, q2[o], q2[o + 1], q2[o + 2]);
+        b[o + 2] = dot3(e3, q2[o], q2[o + 1], q2[o + 2]);
+    }
+    bool none;
+    if constexpr (NSTATE == 3 && FAST) {
+        none = hlld_fp64(a, b, G, SL, SR);
+    } else {
+        double SM;
+        none = (riemann<double, NSTATE, false, false, true, true>(a, b, 0.0, n_disc, G, SL, SR, SM) & kFlagWave) != 0;
+#pragma unroll
+        for (int v = 5; v < 8; v++) G[v] *= kInvSpi4;
+    }
+    F[0] = G[0];
+    F[4] = G[4];
+    // the normal read again and the frame formed again: fewer registers across the solver than
+    // keeping nine doubles
+    double m[3];
+    reload(m);
+    tangent_frame(m, e2, e3);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        F[1 + c] = fma(m[c], G[1], fma(e2[c], G[2], e3[c] * G[3]));
+        F[5 + c] = fma(m[c], G[5], fma(e2[c], G[6], e3[c] * G[7]));
+    }
+    return none;
 }
 
 }  // namespace sb

@@ -373,11 +373,13 @@ void fl_destroy(FaceListDev* f);
 const int32_t* fl_perm(const FaceListDev* f);
 // Uploads the H-atom fluids (Cell_par columns 9..16) of a face list with physics 1; no-op else.
 int fl_set_hatom(FaceListDev* f, const double* cell_par, cudaStream_t s);
-// One stage on the face list: primitive pass, face fluxes (+ dt candidate when want_dt), cell
-// update (kind 0: Euler / Heun stage 1, kind 1: Heun stage 2); a finalizing stage rolls the clock.
+// One stage on the face list: face fluxes (+ dt candidate when want_dt), cell update (kind 0: Euler /
+// Heun stage 1, kind 1: Heun stage 2); a finalizing stage rolls the clock.  `first`: the primitive
+// state is formed from Uin by a pass of its own (the first stage of a call); `more`: another stage of
+// the call follows on Uout, whose primitive state the cell update then leaves for it.
 cudaError_t fl_launch_stage(const FaceListDev* f, const double* Uin, const double* Ubase, double* Uout, int64_t vs,
                             DevClock* clk, DevStatus* st, const setb_step_opts* o, int kind, bool want_dt,
-                            bool finalize, cudaStream_t s);
+                            bool finalize, bool first, bool more, cudaStream_t s);
 
 // ---------------------------------------------------------------- launch entry points
 // kind 0: Euler step / Heun stage 1 (reduces the dt candidate), kind 1: Heun stage 2.
