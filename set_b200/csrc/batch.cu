@@ -30,6 +30,9 @@ namespace {
 
 constexpr int kCheckBlocks = 64;     // fixed partial count per solve: deterministic reduction
 constexpr int kMaxGraphSteps = 64;   // steps captured in one graph
+// Device memory a batch keeps from retired solves (the default pool returns it to the driver at every
+// synchronisation, and mapping a slot anew costs milliseconds).
+constexpr unsigned long long kKeepBytes = 4ull << 30;
 
 struct Slot {
     bool active = false;
@@ -98,6 +101,7 @@ struct setb_batch {
     int precision = 0;
     int sm_count = 148;
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;   // of the slots' memory: keeps up to kKeepBytes of retired solves' for new ones
     int64_t budget = 0, used = 0;
     std::vector<Slot> slots;
     // device arrays
@@ -338,6 +342,20 @@ int32_t setb_batch_create(setb_batch** out, int32_t max_slots, int32_t precision
     b->precision = precision;
     b->budget = hbm_budget;
     b->slots.resize(max_slots);
+    host_pool_acquire();   // released by setb_batch_destroy
+    {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = b->device;
+        unsigned long long keep = kKeepBytes;
+        if (cudaMemPoolCreate(&b->pool, &props) == cudaSuccess) {
+            cudaMemPoolSetAttribute(b->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        } else {   // the device's default pool
+            cudaGetLastError();
+            b->pool = nullptr;
+        }
+    }
     bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess &&
               prepare_batch_kernels(precision) == cudaSuccess &&
               cudaMalloc(&b->d_inst1, sizeof(StageArgs) * max_slots) == cudaSuccess &&
@@ -383,7 +401,8 @@ int32_t setb_batch_add(setb_batch* b, const setb_cart_desc* d, const setb_lism_i
     sl.g = geom_of(d);
     sl.bytes = slot_bytes(sl.g);
     if (b->used + (int64_t)sl.bytes > b->budget) return SETB_EBUSY;
-    if (cudaMallocAsync((void**)&sl.mem, sl.bytes, b->stream) != cudaSuccess) {
+    if ((b->pool ? cudaMallocFromPoolAsync((void**)&sl.mem, sl.bytes, b->pool, b->stream)
+                 : cudaMallocAsync((void**)&sl.mem, sl.bytes, b->stream)) != cudaSuccess) {
         cudaGetLastError();
         return SETB_ENOMEM;
     }
@@ -493,10 +512,11 @@ int32_t setb_batch_get_conserved(setb_batch* b, int32_t slot, double* U) {
     cudaSetDevice(b->device);
     const Slot& sl = b->slots[slot];
     const size_t N = (size_t)sl.g.nx * sl.g.ny * sl.g.nz;
+    RowCopy out[8];
     for (int v = 0; v < 8; v++)
-        SB_TRY(cudaMemcpy2DAsync(U + v * N, sl.g.nx * sizeof(double), sl.U + v * sl.g.vs, sl.g.px * sizeof(double),
-                                 sl.g.nx * sizeof(double), (size_t)sl.g.ny * sl.g.nz, cudaMemcpyDeviceToHost,
-                                 b->stream));
+        out[v] = row_copy_out(U + v * N, sl.g.nx * sizeof(double), sl.U + v * sl.g.vs, sl.g.px * sizeof(double),
+                              sl.g.nx * sizeof(double), (size_t)sl.g.ny * sl.g.nz, nullptr);
+    SB_TRY(copy_rows(out, 8, b->stream));
     SB_TRY(cudaStreamSynchronize(b->stream));
     return SETB_OK;
 }
@@ -635,7 +655,9 @@ int32_t setb_batch_destroy(setb_batch* b) {
     if (b->h_items) cudaFreeHost(b->h_items);
     if (b->h_check_args) cudaFreeHost(b->h_check_args);
     if (b->h_check) cudaFreeHost(b->h_check);
+    if (b->pool) cudaMemPoolDestroy(b->pool);   // every slot has been freed and the stream is idle
     if (b->stream) cudaStreamDestroy(b->stream);
+    host_pool_release();
     delete b;
     return SETB_OK;
 }

@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -203,6 +204,7 @@ void destroy_impl(setb_handle* h) {
     if (h->h_clk) cudaFreeHost(h->h_clk);
     if (h->h_st) cudaFreeHost(h->h_st);
     if (h->stream) cudaStreamDestroy(h->stream);
+    host_pool_release();
     cudaSetDevice(prev);
     delete h;
 }
@@ -225,11 +227,13 @@ int create_impl(setb_handle** out, const setb_cart_desc* d, const GridGeom* geo 
         delete h;
         return SETB_ECUDA;
     }
+    host_pool_acquire();   // released by destroy_impl
     h->sm_count = prop.multiProcessorCount;
     h->ctas_per_sm = tile_shape(0, 0).ctas_per_sm;
     h->g.lz = choose_lz(h->g, h->sm_count, 0, 0);
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
-        delete h;
+        h->stream = nullptr;
+        destroy_impl(h);
         return SETB_ECUDA;
     }
     const size_t bytes = sizeof(double) * 8 * (size_t)h->g.vs;
@@ -283,26 +287,100 @@ int upload_cellpar(setb_handle* h, const double* cell_par) {
         const size_t plane = (size_t)h->g.nx * h->g.ny;
         const size_t own = plane * (size_t)(plane_end(h->g) - plane_begin(h->g));
         SB_TRY(cudaMemsetAsync(stage, 0, sizeof(double) * 8 * N, h->stream));
-        SB_TRY(cudaMemcpy2DAsync(stage + 8 * plane * (size_t)h->g.kb, 8 * sizeof(double), cell_par, 16 * sizeof(double),
-                                 8 * sizeof(double), own, cudaMemcpyHostToDevice, h->stream));
+        SB_TRY(copy_rows_to_device(stage + 8 * plane * (size_t)h->g.kb, cell_par, 16 * sizeof(double),
+                                   8 * sizeof(double), own, nullptr, h->stream));
         SB_TRY(launch_prim_to_cons(h->g, stage, h->buf[h->cur], h->stream));
         return SETB_OK;
     }
     if (const int32_t* perm = fl_perm(h->fl)) {
         const int rc = fl_set_hatom(h->fl, cell_par, h->stream);
         if (rc) return rc;
-        std::vector<double> tmp(8 * N);
-        for (size_t d = 0; d < N; d++) std::memcpy(&tmp[8 * d], cell_par + 16 * (size_t)perm[d], 8 * sizeof(double));
-        SB_TRY(cudaMemcpyAsync(stage, tmp.data(), sizeof(double) * 8 * N, cudaMemcpyHostToDevice, h->stream));
+        SB_TRY(copy_rows_to_device(stage, cell_par, 16 * sizeof(double), 8 * sizeof(double), N, perm, h->stream));
         SB_TRY(launch_prim_to_cons(h->g, stage, h->buf[h->cur], h->stream));
-        SB_TRY(cudaStreamSynchronize(h->stream));   // tmp is released on return
         return SETB_OK;
     }
-    SB_TRY(cudaMemcpy2DAsync(stage, 8 * sizeof(double), cell_par, 16 * sizeof(double), 8 * sizeof(double), N,
-                             cudaMemcpyHostToDevice, h->stream));
+    SB_TRY(copy_rows_to_device(stage, cell_par, 16 * sizeof(double), 8 * sizeof(double), N, nullptr, h->stream));
     SB_TRY(launch_prim_to_cons(h->g, stage, h->buf[h->cur], h->stream));
     return SETB_OK;
 }
+
+// Device memory of one flux call on host arrays: a stream and one block from a memory pool per device
+// that keeps at most 64 MB between calls (eight cudaMalloc / cudaFree pairs a call cost ~1 ms).  The
+// pool is stream-ordered, so calls from several threads do not see each other's blocks.
+cudaMemPool_t flux_pool(int device) {
+    constexpr int kMaxDevices = 64;
+    static std::mutex mu;
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    if (device < 0 || device >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!pools[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        unsigned long long keep = 64ull << 20;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[device] = p;
+    }
+    return pools[device];
+}
+
+struct FluxBlock {
+    int rc = SETB_OK;
+    cudaStream_t s = nullptr;
+    int32_t* flags = nullptr;
+    FluxBlock(size_t n_doubles, size_t n_flags) : nf(n_flags) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaGetLastError();
+            s = nullptr;
+            rc = SETB_ECUDA;
+            return;
+        }
+        const size_t bytes = n_doubles * sizeof(double) + n_flags * sizeof(int32_t);
+        cudaMemPool_t p = flux_pool(dev);
+        if ((p ? cudaMallocFromPoolAsync((void**)&mem, bytes, p, s) : cudaMallocAsync((void**)&mem, bytes, s)) != cudaSuccess) {
+            cudaGetLastError();
+            mem = nullptr;
+            rc = SETB_ENOMEM;
+            return;
+        }
+        at = mem;
+        flags = reinterpret_cast<int32_t*>(mem + n_doubles);
+    }
+    ~FluxBlock() {
+        if (mem) cudaFreeAsync(mem, s);
+        if (s) cudaStreamDestroy(s);   // frees its resources once its work is done
+    }
+    FluxBlock(const FluxBlock&) = delete;
+    FluxBlock& operator=(const FluxBlock&) = delete;
+    double* doubles(size_t k) {
+        double* p = at;
+        at += k;
+        return p;
+    }
+    // k doubles from / to a host array (nullptr: none)
+    RowCopy up(double* d, const double* h, size_t k) const { return row_copy_in(d, h, kRow, kRow, h ? k : 0, nullptr); }
+    RowCopy down(double* h, const double* d, size_t k) const {
+        return row_copy_out(h, kRow, d, kRow, kRow, h ? k : 0, nullptr);
+    }
+    RowCopy flags_down(int32_t* h) const { return row_copy_out(h, 4, flags, 4, 4, nf, nullptr); }
+    int finish(bool ok) {
+        if (cudaStreamSynchronize(s) != cudaSuccess) ok = false;
+        if (!ok) cudaGetLastError();
+        return ok ? SETB_OK : SETB_ECUDA;
+    }
+
+private:
+    static constexpr size_t kRow = sizeof(double);
+    double *mem = nullptr, *at = nullptr;
+    size_t nf;
+};
 
 template <typename T, int NS>
 void chlld_host(const double* n, double w, const double* q1, const double* q2, int n_disc, double* qqq,
@@ -389,42 +467,19 @@ int32_t setb_chlld_q_batch(int64_t n, int32_t n_state, int32_t n_disc, int32_t y
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return SETB_ENODEV;
     const size_t sn = (size_t)n;
-    double *dn = nullptr, *dw = nullptr, *d1 = nullptr, *d2 = nullptr, *dk = nullptr, *dq = nullptr, *ds = nullptr;
-    int32_t* df = nullptr;
-    cudaStream_t s = nullptr;
-    int rc = SETB_OK;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return SETB_ECUDA;
-    if (cudaMalloc(&dn, 3 * sn * 8) || (w && cudaMalloc(&dw, sn * 8)) || cudaMalloc(&d1, 9 * sn * 8) ||
-        cudaMalloc(&d2, 9 * sn * 8) || (konvect && cudaMalloc(&dk, 3 * sn * 8)) || cudaMalloc(&dq, 9 * sn * 8) ||
-        cudaMalloc(&ds, 3 * sn * 8) || cudaMalloc(&df, sn * 4)) {
-        cudaGetLastError();
-        rc = SETB_ENOMEM;
-    }
-    if (rc == SETB_OK) {
-        bool ok = cudaMemcpyAsync(dn, normals, 3 * sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                  (!w || cudaMemcpyAsync(dw, w, sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess) &&
-                  cudaMemcpyAsync(d1, q1, 9 * sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                  cudaMemcpyAsync(d2, q2, 9 * sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                  (!konvect || cudaMemcpyAsync(dk, konvect, 3 * sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess) &&
-                  launch_chlld_q_batch(n, n_state, n_disc, ydar != 0, dn, dw, d1, d2, dk, dq, ds, df, s) ==
-                      cudaSuccess &&
-                  cudaMemcpyAsync(qqq, dq, 9 * sn * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                  cudaMemcpyAsync(speeds, ds, 3 * sn * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                  cudaMemcpyAsync(flags, df, sn * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                  (!konvect || cudaMemcpyAsync(konvect, dk, 3 * sn * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess) &&
-                  cudaStreamSynchronize(s) == cudaSuccess;
-        if (!ok) rc = SETB_ECUDA;
-    }
-    cudaFree(dn);
-    cudaFree(dw);
-    cudaFree(d1);
-    cudaFree(d2);
-    cudaFree(dk);
-    cudaFree(dq);
-    cudaFree(ds);
-    cudaFree(df);
-    cudaStreamDestroy(s);
-    return rc;
+    FluxBlock blk(3 * sn + (w ? sn : 0) + 9 * sn + 9 * sn + (konvect ? 3 * sn : 0) + 9 * sn + 3 * sn, sn);
+    if (blk.rc) return blk.rc;
+    double *dn = blk.doubles(3 * sn), *dw = w ? blk.doubles(sn) : nullptr, *d1 = blk.doubles(9 * sn),
+           *d2 = blk.doubles(9 * sn), *dk = konvect ? blk.doubles(3 * sn) : nullptr, *dq = blk.doubles(9 * sn),
+           *ds = blk.doubles(3 * sn);
+    const RowCopy in[] = {blk.up(dn, normals, 3 * sn), blk.up(dw, w, sn), blk.up(d1, q1, 9 * sn),
+                          blk.up(d2, q2, 9 * sn), blk.up(dk, konvect, 3 * sn)};
+    const RowCopy out[] = {blk.down(qqq, dq, 9 * sn), blk.down(speeds, ds, 3 * sn), blk.down(konvect, dk, 3 * sn),
+                           blk.flags_down(flags)};
+    return blk.finish(copy_rows(in, 5, blk.s) == cudaSuccess &&
+                      launch_chlld_q_batch(n, n_state, n_disc, ydar != 0, dn, dw, d1, d2, dk, dq, ds, blk.flags,
+                                           blk.s) == cudaSuccess &&
+                      copy_rows(out, 4, blk.s) == cudaSuccess);
 }
 
 int32_t setb_chlld_batch(int64_t n, int32_t n_state, int32_t n_disc, int32_t precision, const double* normals,
@@ -437,39 +492,17 @@ int32_t setb_chlld_batch(int64_t n, int32_t n_state, int32_t n_disc, int32_t pre
     if (!normals || !q1 || !q2 || !qqq || !speeds || !flags) return SETB_EINVAL;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return SETB_ENODEV;
-    double *dn = nullptr, *dw = nullptr, *d1 = nullptr, *d2 = nullptr, *dq = nullptr, *ds = nullptr;
-    int32_t* df = nullptr;
-    cudaStream_t s = nullptr;
-    int rc = SETB_OK;
     const size_t sn = (size_t)n;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return SETB_ECUDA;
-    if (cudaMalloc(&dn, 3 * sn * 8) || (w && cudaMalloc(&dw, sn * 8)) || cudaMalloc(&d1, 8 * sn * 8) ||
-        cudaMalloc(&d2, 8 * sn * 8) || cudaMalloc(&dq, 8 * sn * 8) || cudaMalloc(&ds, 3 * sn * 8) ||
-        cudaMalloc(&df, sn * 4)) {
-        cudaGetLastError();
-        rc = SETB_ENOMEM;
-    }
-    if (rc == SETB_OK) {
-        bool ok = cudaMemcpyAsync(dn, normals, 3 * sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                  (!w || cudaMemcpyAsync(dw, w, sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess) &&
-                  cudaMemcpyAsync(d1, q1, 8 * sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                  cudaMemcpyAsync(d2, q2, 8 * sn * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-                  launch_chlld_batch(n, n_state, n_disc, precision, dn, dw, d1, d2, dq, ds, df, s) == cudaSuccess &&
-                  cudaMemcpyAsync(qqq, dq, 8 * sn * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                  cudaMemcpyAsync(speeds, ds, 3 * sn * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                  cudaMemcpyAsync(flags, df, sn * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                  cudaStreamSynchronize(s) == cudaSuccess;
-        if (!ok) rc = SETB_ECUDA;
-    }
-    cudaFree(dn);
-    cudaFree(dw);
-    cudaFree(d1);
-    cudaFree(d2);
-    cudaFree(dq);
-    cudaFree(ds);
-    cudaFree(df);
-    cudaStreamDestroy(s);
-    return rc;
+    FluxBlock blk(3 * sn + (w ? sn : 0) + 8 * sn + 8 * sn + 8 * sn + 3 * sn, sn);
+    if (blk.rc) return blk.rc;
+    double *dn = blk.doubles(3 * sn), *dw = w ? blk.doubles(sn) : nullptr, *d1 = blk.doubles(8 * sn),
+           *d2 = blk.doubles(8 * sn), *dq = blk.doubles(8 * sn), *ds = blk.doubles(3 * sn);
+    const RowCopy in[] = {blk.up(dn, normals, 3 * sn), blk.up(dw, w, sn), blk.up(d1, q1, 8 * sn), blk.up(d2, q2, 8 * sn)};
+    const RowCopy out[] = {blk.down(qqq, dq, 8 * sn), blk.down(speeds, ds, 3 * sn), blk.flags_down(flags)};
+    return blk.finish(copy_rows(in, 4, blk.s) == cudaSuccess &&
+                      launch_chlld_batch(n, n_state, n_disc, precision, dn, dw, d1, d2, dq, ds, blk.flags, blk.s) ==
+                          cudaSuccess &&
+                      copy_rows(out, 3, blk.s) == cudaSuccess);
 }
 
 int32_t setb_cart_fill_lism(const setb_cart_desc* d, const setb_lism_ic* ic, double* cell_par) {
@@ -752,15 +785,13 @@ int32_t setb_get_state(setb_handle* h, double* cell_par, double* time_all) {
     double* stage = h->buf[1 - h->cur];
     SB_TRY(launch_cons_to_prim(h->g, h->buf[h->cur], stage, h->stream));
     if (const int32_t* perm = fl_perm(h->fl)) {
-        std::vector<double> tmp(8 * N);
-        SB_TRY(cudaMemcpyAsync(tmp.data(), stage, sizeof(double) * 8 * N, cudaMemcpyDeviceToHost, h->stream));
-        SB_TRY(cudaStreamSynchronize(h->stream));
-        for (size_t d = 0; d < N; d++) std::memcpy(cell_par + 16 * (size_t)perm[d], &tmp[8 * d], 8 * sizeof(double));
+        SB_TRY(copy_rows_to_host(cell_par, 16 * sizeof(double), stage, 8 * sizeof(double), 8 * sizeof(double), N, perm,
+                                 h->stream));
     } else {
         const size_t plane = (size_t)h->g.nx * h->g.ny;   // a z slab returns its owned planes
         const size_t own = plane * (size_t)(plane_end(h->g) - plane_begin(h->g));
-        SB_TRY(cudaMemcpy2DAsync(cell_par, 16 * sizeof(double), stage + 8 * plane * (size_t)h->g.kb,
-                                 8 * sizeof(double), 8 * sizeof(double), own, cudaMemcpyDeviceToHost, h->stream));
+        SB_TRY(copy_rows_to_host(cell_par, 16 * sizeof(double), stage + 8 * plane * (size_t)h->g.kb,
+                                 8 * sizeof(double), 8 * sizeof(double), own, nullptr, h->stream));
     }
     int rc = download_clock(h);
     if (rc) return rc;
@@ -809,16 +840,15 @@ int32_t setb_get_conserved(setb_handle* h, double* U) {
     const int nown = plane_end(h->g) - plane_begin(h->g);   // a z slab returns its owned planes
     const size_t N = (size_t)h->g.nx * h->g.ny * nown;
     const int32_t* perm = fl_perm(h->fl);
-    std::vector<double> tmp(perm ? 8 * N : 0);
-    double* dst = perm ? tmp.data() : U;
-    for (int v = 0; v < 8; v++)
-        SB_TRY(cudaMemcpy2DAsync(dst + v * N, h->g.nx * sizeof(double),
-                                 h->buf[h->cur] + v * h->g.vs + (long long)h->g.kb * h->g.ps, h->g.px * sizeof(double),
-                                 h->g.nx * sizeof(double), (size_t)h->g.ny * nown, cudaMemcpyDeviceToHost, h->stream));
+    RowCopy out[8];
+    for (int v = 0; v < 8; v++) {
+        const double* src = h->buf[h->cur] + v * h->g.vs + (long long)h->g.kb * h->g.ps;
+        out[v] = perm ? row_copy_out(U + v * N, sizeof(double), src, sizeof(double), sizeof(double), N, perm)
+                      : row_copy_out(U + v * N, h->g.nx * sizeof(double), src, h->g.px * sizeof(double),
+                                     h->g.nx * sizeof(double), (size_t)h->g.ny * nown, nullptr);
+    }
+    SB_TRY(copy_rows(out, 8, h->stream));
     SB_TRY(cudaStreamSynchronize(h->stream));
-    if (perm)
-        for (int v = 0; v < 8; v++)
-            for (size_t d = 0; d < N; d++) U[v * N + (size_t)perm[d]] = tmp[v * N + d];
     return SETB_OK;
 }
 

@@ -745,11 +745,8 @@ namespace sb {
 // Uploads the H-atom fluids (Cell_par columns 9..16, caller numbering) of a physics-1 face list.
 int fl_set_hatom(FaceListDev* f, const double* cell_par, cudaStream_t s) {
     if (!f || !f->v.hatom) return SETB_OK;
-    const size_t N = (size_t)f->v.n_cell;
-    std::vector<double> tmp(8 * N);
-    for (size_t d = 0; d < N; d++) std::memcpy(&tmp[8 * d], cell_par + 16 * (size_t)f->perm[d] + 8, 8 * sizeof(double));
-    if (cudaMemcpyAsync(f->v.hatom, tmp.data(), sizeof(double) * 8 * N, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
+    if (copy_rows_to_device(f->v.hatom, cell_par + 8, 16 * sizeof(double), 8 * sizeof(double), (size_t)f->v.n_cell,
+                            f->perm.data(), s) != cudaSuccess)
         return SETB_ECUDA;
     return SETB_OK;
 }

@@ -9,10 +9,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
-#include <vector>
 
 #include "setb_internal.cuh"
 
@@ -21,29 +20,23 @@ namespace {
 
 constexpr size_t kSlotBytes = 512 << 10;
 constexpr int kMaxThreads = 8;
-// Slots kept for later transfers: 8 MiB of pinned memory at most, freed when no handle or batch is
-// left (host_pool_release).  Transfers that overlap take more and give them back to the driver.
-constexpr size_t kKeepSlots = 2 * kMaxThreads;
+// Slots kept for later transfers: 8 MiB of pinned memory at most, given back when the last handle or
+// batch goes (host_pool_release; a program that makes flux calls alone keeps them).  Transfers that
+// overlap take more and give them back at once.
+constexpr int kKeepSlots = 2 * kMaxThreads;
 
 struct Pool {
     std::mutex mu;
-    std::vector<void*> free;
+    void* free[kKeepSlots] = {};
+    int n = 0;
     long long owners = 0;
 };
-Pool& pool() {
-    static Pool* p = new Pool;   // never destroyed: calls may come from other threads at exit
-    return *p;
-}
+Pool g_pool;
 
 void* take_slot() {
-    Pool& p = pool();
     {
-        std::lock_guard<std::mutex> lock(p.mu);
-        if (!p.free.empty()) {
-            void* s = p.free.back();
-            p.free.pop_back();
-            return s;
-        }
+        std::lock_guard<std::mutex> lock(g_pool.mu);
+        if (g_pool.n > 0) return g_pool.free[--g_pool.n];
     }
     void* s = nullptr;
     if (cudaHostAlloc(&s, kSlotBytes, cudaHostAllocPortable) != cudaSuccess) {
@@ -55,11 +48,10 @@ void* take_slot() {
 
 void give_slot(void* s) {
     if (!s) return;
-    Pool& p = pool();
     {
-        std::lock_guard<std::mutex> lock(p.mu);
-        if (p.free.size() < kKeepSlots && p.free.capacity() >= kKeepSlots) {
-            p.free.push_back(s);
+        std::lock_guard<std::mutex> lock(g_pool.mu);
+        if (g_pool.n < kKeepSlots) {
+            g_pool.free[g_pool.n++] = s;
             return;
         }
     }
@@ -75,16 +67,14 @@ bool pageable(const void* p) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-struct Rows {
-    bool to_device;
-    char* dev;
-    size_t dpitch;
-    char* host;
-    size_t hpitch, width, n;
-    const int32_t* perm;
+// The copies of one call, handed out in slot-sized chunks.
+struct Team {
+    const RowCopy* copy[kMaxRowCopies];
+    size_t per[kMaxRowCopies];         // rows of a slot
+    size_t end[kMaxRowCopies];         // chunks up to and including this copy
+    int n = 0;
     cudaStream_t stream;
-    size_t per;                    // rows of a slot
-    std::atomic<size_t> next{0};   // next chunk
+    std::atomic<size_t> next{0};
     std::atomic<int> err{0};
 };
 
@@ -96,19 +86,20 @@ void move_fixed(char* slot, size_t sp, char* host, size_t hp, size_t r0, size_t 
         else std::memcpy(h, slot + sp * r, W);
     }
 }
-// Rows r0 .. r0 + m between a slot (row pitch `sp`) and host memory; `in`: into the slot.
-void move_rows(const Rows& t, char* slot, size_t r0, size_t m, bool in) {
+// Rows r0 .. r0 + m between a slot (row pitch as the device's) and host memory; `in`: into the slot.
+void move_rows(const RowCopy& t, char* slot, size_t r0, size_t m, bool in) {
+    char* host = static_cast<char*>(t.host);
     const size_t sp = t.dpitch;
     if (!t.perm && t.hpitch == t.width && sp == t.width) {
-        if (in) std::memcpy(slot, t.host + t.width * r0, t.width * m);
-        else std::memcpy(t.host + t.width * r0, slot, t.width * m);
+        if (in) std::memcpy(slot, host + t.width * r0, t.width * m);
+        else std::memcpy(host + t.width * r0, slot, t.width * m);
     } else if (t.width == 64) {
-        move_fixed<64>(slot, sp, t.host, t.hpitch, r0, m, t.perm, in);
+        move_fixed<64>(slot, sp, host, t.hpitch, r0, m, t.perm, in);
     } else if (t.width == 8) {
-        move_fixed<8>(slot, sp, t.host, t.hpitch, r0, m, t.perm, in);
+        move_fixed<8>(slot, sp, host, t.hpitch, r0, m, t.perm, in);
     } else {
         for (size_t r = 0; r < m; r++) {
-            char* h = t.host + t.hpitch * (t.perm ? (size_t)t.perm[r0 + r] : r0 + r);
+            char* h = host + t.hpitch * (t.perm ? (size_t)t.perm[r0 + r] : r0 + r);
             if (in) std::memcpy(slot + sp * r, h, t.width);
             else std::memcpy(h, slot + sp * r, t.width);
         }
@@ -116,38 +107,42 @@ void move_rows(const Rows& t, char* slot, size_t r0, size_t m, bool in) {
 }
 
 // One thread's share: two slots, so one is gathered or scattered while the other's copy runs.
-void work(Rows* t, int device, void* s0, void* s1) {
+void work(Team* t, int device, void* s0, void* s1) {
     cudaError_t e = cudaSetDevice(device);
     char* slot[2] = {static_cast<char*>(s0), static_cast<char*>(s1)};
     cudaEvent_t ev[2] = {nullptr, nullptr};
     for (int b = 0; b < 2 && e == cudaSuccess; b++) e = cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming);
-    size_t first[2] = {0, 0}, count[2] = {0, 0};   // rows in flight in each slot
-    const size_t chunks = (t->n + t->per - 1) / t->per;
+    const RowCopy* which[2] = {nullptr, nullptr};   // rows in flight in each slot
+    size_t first[2] = {0, 0}, count[2] = {0, 0};
     bool more = true;
     for (int b = 0; e == cudaSuccess && t->err.load() == 0; b ^= 1) {
         if (count[b]) {
             e = cudaEventSynchronize(ev[b]);
             if (e != cudaSuccess) break;
-            if (!t->to_device) move_rows(*t, slot[b], first[b], count[b], false);
+            if (!which[b]->to_device) move_rows(*which[b], slot[b], first[b], count[b], false);
             count[b] = 0;
         }
-        const size_t c = more ? t->next.fetch_add(1) : chunks;
-        if (c >= chunks) {
+        size_t c = more ? t->next.fetch_add(1) : t->end[t->n - 1];
+        if (c >= t->end[t->n - 1]) {
             more = false;
             if (!count[b ^ 1]) break;
             continue;
         }
-        const size_t r0 = c * t->per, m = std::min(t->per, t->n - r0);
-        char* d = t->dev + t->dpitch * r0;
-        // the last row of the device's rows may end at its payload
-        const size_t bytes = t->dpitch * (m - 1) + t->width;
-        if (t->to_device) {
-            move_rows(*t, slot[b], r0, m, true);
-            e = cudaMemcpyAsync(d, slot[b], bytes, cudaMemcpyHostToDevice, t->stream);
+        int k = 0;
+        while (c >= t->end[k]) k++;
+        if (k) c -= t->end[k - 1];
+        const RowCopy& y = *t->copy[k];
+        const size_t r0 = c * t->per[k], m = std::min(t->per[k], y.n - r0);
+        char* dev = static_cast<char*>(y.dev) + y.dpitch * r0;
+        const size_t bytes = y.dpitch * (m - 1) + y.width;   // the last row may end at its payload
+        if (y.to_device) {
+            move_rows(y, slot[b], r0, m, true);
+            e = cudaMemcpyAsync(dev, slot[b], bytes, cudaMemcpyHostToDevice, t->stream);
         } else {
-            e = cudaMemcpyAsync(slot[b], d, bytes, cudaMemcpyDeviceToHost, t->stream);
+            e = cudaMemcpyAsync(slot[b], dev, bytes, cudaMemcpyDeviceToHost, t->stream);
         }
         if (e == cudaSuccess) e = cudaEventRecord(ev[b], t->stream);
+        which[b] = &y;
         first[b] = r0;
         count[b] = m;
     }
@@ -156,20 +151,56 @@ void work(Rows* t, int device, void* s0, void* s1) {
         if (ev[b]) cudaEventDestroy(ev[b]);
 }
 
-cudaError_t run_rows(Rows& t) {
-    if (t.n == 0) return cudaSuccess;
-    const size_t total = t.n * t.width;
-    const bool direct = t.perm == nullptr && (total < (64u << 10) || t.dpitch > kSlotBytes || !pageable(t.host));
-    if (direct) {
-        if (t.to_device)
-            return cudaMemcpy2DAsync(t.dev, t.dpitch, t.host, t.hpitch, t.width, t.n, cudaMemcpyHostToDevice, t.stream);
-        return cudaMemcpy2DAsync(t.host, t.hpitch, t.dev, t.dpitch, t.width, t.n, cudaMemcpyDeviceToHost, t.stream);
+// A copy the driver makes by itself: known memory, or too little to be worth a slot.
+bool is_direct(const RowCopy& c) {
+    return !c.perm && (c.n * c.width < (64u << 10) || c.dpitch > kSlotBytes || !pageable(c.host));
+}
+
+}  // namespace
+
+void host_pool_acquire() {
+    std::lock_guard<std::mutex> lock(g_pool.mu);
+    g_pool.owners++;
+}
+
+void host_pool_release() {
+    void* drop[kKeepSlots];
+    int n = 0;
+    {
+        std::lock_guard<std::mutex> lock(g_pool.mu);
+        if (--g_pool.owners == 0)
+            for (; g_pool.n > 0; n++) drop[n] = g_pool.free[--g_pool.n];
     }
-    t.per = std::max<size_t>(1, kSlotBytes / t.dpitch);
+    for (int k = 0; k < n; k++) cudaFreeHost(drop[k]);
+}
+
+cudaError_t copy_rows(const RowCopy* list, int count, cudaStream_t s) {
+    Team t;
+    t.stream = s;
+    size_t total = 0, chunks = 0;
+    for (int k = 0; k < count; k++) {
+        const RowCopy& c = list[k];
+        if (c.n == 0) continue;
+        if (c.to_device && c.dpitch != c.width) return cudaErrorInvalidValue;   // would write its row padding
+        if (is_direct(c)) {
+            const cudaError_t e =
+                c.to_device ? cudaMemcpy2DAsync(c.dev, c.dpitch, c.host, c.hpitch, c.width, c.n, cudaMemcpyHostToDevice, s)
+                            : cudaMemcpy2DAsync(c.host, c.hpitch, c.dev, c.dpitch, c.width, c.n, cudaMemcpyDeviceToHost, s);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
+        if (t.n == kMaxRowCopies) return cudaErrorInvalidValue;
+        t.copy[t.n] = &c;
+        t.per[t.n] = std::max<size_t>(1, kSlotBytes / c.dpitch);
+        chunks += (c.n + t.per[t.n] - 1) / t.per[t.n];
+        t.end[t.n++] = chunks;
+        total += c.n * c.width;
+    }
+    if (t.n == 0) return cudaSuccess;
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    const int hw = std::max(1u, std::thread::hardware_concurrency());
+    const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
     const int want = (int)std::min<size_t>(std::min(kMaxThreads, hw), (total + (1u << 20) - 1) >> 20);
     void* slots[2 * kMaxThreads] = {};
     int pairs = 0;
@@ -187,69 +218,29 @@ cudaError_t run_rows(Rows& t) {
             try {
                 th[started] = std::thread(work, &t, device, slots[2 * k], slots[2 * k + 1]);
                 started++;
-            } catch (const std::system_error&) {   // no more threads: the others take its chunks
+            } catch (const std::exception&) {   // no more threads: the others take its chunks
                 break;
             }
         }
         work(&t, device, slots[0], slots[1]);
         for (int k = 0; k < started; k++) th[k].join();
         e = (cudaError_t)t.err.load();
-        if (e != cudaSuccess) cudaStreamSynchronize(t.stream);   // no copy may still use a slot
+        if (e != cudaSuccess) cudaStreamSynchronize(s);   // no copy may still use a slot
     }
-    for (void* s : slots) give_slot(s);
+    for (void* p : slots) give_slot(p);
     return e;
-}
-
-}  // namespace
-
-void host_pool_acquire() {
-    Pool& p = pool();
-    std::lock_guard<std::mutex> lock(p.mu);
-    p.owners++;
-    try {
-        p.free.reserve(kKeepSlots);
-    } catch (const std::bad_alloc&) {   // nothing is kept then (give_slot)
-    }
-}
-
-void host_pool_release() {
-    std::vector<void*> drop;
-    Pool& p = pool();
-    {
-        std::lock_guard<std::mutex> lock(p.mu);
-        if (--p.owners == 0) drop.swap(p.free);
-    }
-    for (void* s : drop) cudaFreeHost(s);
 }
 
 cudaError_t copy_rows_to_device(void* dev, const void* host, size_t hpitch, size_t width, size_t n,
                                 const int32_t* perm, cudaStream_t s) {
-    Rows t;
-    t.to_device = true;
-    t.dev = static_cast<char*>(dev);
-    t.dpitch = width;
-    t.host = const_cast<char*>(static_cast<const char*>(host));   // read only
-    t.hpitch = hpitch;
-    t.width = width;
-    t.n = n;
-    t.perm = perm;
-    t.stream = s;
-    return run_rows(t);
+    const RowCopy c = row_copy_in(dev, host, hpitch, width, n, perm);
+    return copy_rows(&c, 1, s);
 }
 
 cudaError_t copy_rows_to_host(void* host, size_t hpitch, const void* dev, size_t dpitch, size_t width, size_t n,
                               const int32_t* perm, cudaStream_t s) {
-    Rows t;
-    t.to_device = false;
-    t.dev = const_cast<char*>(static_cast<const char*>(dev));     // read only
-    t.dpitch = dpitch;
-    t.host = static_cast<char*>(host);
-    t.hpitch = hpitch;
-    t.width = width;
-    t.n = n;
-    t.perm = perm;
-    t.stream = s;
-    return run_rows(t);
+    const RowCopy c = row_copy_out(host, hpitch, dev, dpitch, width, n, perm);
+    return copy_rows(&c, 1, s);
 }
 
 }  // namespace sb

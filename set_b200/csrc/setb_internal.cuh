@@ -381,6 +381,35 @@ cudaError_t fl_launch_stage(const FaceListDev* f, const double* Uin, const doubl
                             DevClock* clk, DevStatus* st, const setb_step_opts* o, int kind, bool want_dt,
                             bool finalize, bool first, bool more, cudaStream_t s);
 
+// ---------------------------------------------------------------- host rows (hostpipe.cu)
+// n rows of `width` bytes between host memory (row perm ? perm[r] : r at host + row * hpitch) and the
+// device (row r at dev + r * dpitch), on the calling device.  copy_rows_to_device: packed device rows;
+// the host rows may be reused on return.  copy_rows_to_host: the rows are complete after a
+// synchronisation of `s`.  Calls from several threads and on several streams are independent.
+// copy_rows: several of them by one team of threads, in one direction or both.
+struct RowCopy {
+    bool to_device;
+    void *dev, *host;          // the source side is only read
+    size_t dpitch, hpitch, width, n;
+    const int32_t* perm;
+};
+constexpr int kMaxRowCopies = 16;
+inline RowCopy row_copy_in(void* dev, const void* host, size_t hpitch, size_t width, size_t n, const int32_t* perm) {
+    return RowCopy{true, dev, const_cast<void*>(host), width, hpitch, width, n, perm};
+}
+inline RowCopy row_copy_out(void* host, size_t hpitch, const void* dev, size_t dpitch, size_t width, size_t n,
+                            const int32_t* perm) {
+    return RowCopy{false, const_cast<void*>(dev), host, dpitch, hpitch, width, n, perm};
+}
+cudaError_t copy_rows(const RowCopy* list, int count, cudaStream_t s);
+cudaError_t copy_rows_to_device(void* dev, const void* host, size_t hpitch, size_t width, size_t n,
+                                const int32_t* perm, cudaStream_t s);
+cudaError_t copy_rows_to_host(void* host, size_t hpitch, const void* dev, size_t dpitch, size_t width, size_t n,
+                              const int32_t* perm, cudaStream_t s);
+// Owners of the pinned slots kept between transfers (handles and batches).
+void host_pool_acquire();
+void host_pool_release();
+
 // ---------------------------------------------------------------- launch entry points
 // kind 0: Euler step / Heun stage 1 (reduces the dt candidate), kind 1: Heun stage 2.
 cudaError_t launch_stage(const StageArgs& a, int precision, int n_state, int order, int kind, cudaStream_t s);
