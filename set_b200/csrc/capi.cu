@@ -41,7 +41,6 @@ struct setb_handle {
     CUtensorMap* tmap = nullptr;           // device: [buffer 0/1][tile shape, kShapeTy]
     bool tma_ok[3] = {false, false, false};   // per tile shape: maps encoded (else plain loads)
     FaceListDev* fl = nullptr;             // face-list grid (g is then 1-D: nx = N cells)
-    int ctas_per_sm = 1;
     int sm_count = 148;
     long long copy_wait = 0;               // StageArgs::copy_wait of this handle's launches
 };
@@ -109,17 +108,12 @@ GridGeom make_geom(const setb_cart_desc* d) {
     return g;
 }
 
-// The tile heights a handle keeps tensor maps for (plain, mixed stage 2, mixed stage 1 / delta),
-// and which one a launch uses.
+// The tile heights a handle keeps tensor maps for: the plain / delta form's and the mixed form's two.
 constexpr int kNumShapes = 3;
-constexpr int kShapeTy[kNumShapes] = {tile_shape(0, 0).ty, tile_shape(1, 1).ty, tile_shape(1, 0).ty};
-constexpr bool shape_listed(int ty) { return ty == kShapeTy[0] || ty == kShapeTy[1] || ty == kShapeTy[2]; }
-static_assert(shape_listed(tile_shape(0, 1).ty) && shape_listed(tile_shape(2, 0).ty) && shape_listed(tile_shape(2, 1).ty),
+constexpr int kShapeTy[kNumShapes] = {tile_shape(0, 0).ty, tile_shape(1, 0).ty, tile_shape(1, 1).ty};
+static_assert(tile_shape(2, 0).ty == kShapeTy[0] && num_shapes(0) == 1 && num_shapes(1) == 2 && num_shapes(2) == 1,
               "every stage launch's tile height has a tensor map");
-int shape_index(int precision, int kind) {
-    const int ty = tile_shape(precision, kind).ty;
-    return ty == kShapeTy[0] ? 0 : (ty == kShapeTy[1] ? 1 : 2);
-}
+int shape_index(int precision, int shape) { return precision == 1 ? 1 + shape : 0; }
 
 }  // namespace
 
@@ -128,24 +122,27 @@ int shape_index(int precision, int kind) {
 // march, measured 16 us beside 5.5 us a plane on grids of one wave).  Chunks go down to one plane:
 // a small grid has too few columns for the SMs, and shorter marches cost more work but less time
 // (32^3 a stage 56 us at 8 planes, 22 us at one; 64^3 59 us at 8, 49 us at 6).
-int sb::choose_lz(const GridGeom& g, int sm_count, int precision, int kind) {
-    const TileShape ts = tile_shape(precision, kind);
-    const long long cols = (long long)((g.nx + kTileX - 1) / kTileX) * ((g.ny + ts.ty - 1) / ts.ty);
-    const long long slots = (long long)sm_count * std::max(ts.ctas_per_sm, 1);
+// Among shapes, the one whose padded tiles take least time (interval: their relative cost).
+Tiling sb::choose_tiling(const GridGeom& g, int sm_count, int precision) {
     const int nz = plane_end(g) - plane_begin(g);   // planes the stage kernels update
     double best = 1e300;
-    int best_lz = nz;
-    for (int c = 1; c <= nz; c++) {
-        const int lz = (nz + c - 1) / c;
-        const long long ctas = cols * ((nz + lz - 1) / lz);
-        const long long waves = (ctas + slots - 1) / slots;
-        const double cost = (double)waves * (lz + 3);
-        if (cost < best - 1e-9) {
-            best = cost;
-            best_lz = lz;
+    Tiling t{0, nz};
+    for (int shape = 0; shape < num_shapes(precision); shape++) {
+        const TileShape ts = tile_shape(precision, shape);
+        const long long cols = (long long)((g.nx + kTileX - 1) / kTileX) * ((g.ny + ts.ty - 1) / ts.ty);
+        const long long slots = (long long)sm_count * ts.ctas_per_sm;
+        for (int c = 1; c <= nz; c++) {
+            const int lz = (nz + c - 1) / c;
+            const long long ctas = cols * ((nz + lz - 1) / lz);
+            const long long waves = (ctas + slots - 1) / slots;
+            const double cost = (double)waves * (lz + 3) * ts.interval;
+            if (cost < best - 1e-9) {
+                best = cost;
+                t = Tiling{shape, lz};
+            }
         }
     }
-    return best_lz;
+    return t;
 }
 
 namespace {
@@ -229,8 +226,6 @@ int create_impl(setb_handle** out, const setb_cart_desc* d, const GridGeom* geo 
     }
     host_pool_acquire();   // released by destroy_impl
     h->sm_count = prop.multiProcessorCount;
-    h->ctas_per_sm = tile_shape(0, 0).ctas_per_sm;
-    h->g.lz = choose_lz(h->g, h->sm_count, 0, 0);
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
         h->stream = nullptr;
         destroy_impl(h);
@@ -661,7 +656,9 @@ int enqueue_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaE
     StageArgs a{};
     a.g = h->g;
     const int P = o->precision;
-    const int lz0 = choose_lz(h->g, h->sm_count, P, 0), lz1 = choose_lz(h->g, h->sm_count, P, 1);
+    const Tiling tiling = choose_tiling(h->g, h->sm_count, P);
+    a.g.lz = tiling.lz;
+    a.shape = tiling.shape;
     float* comp = nullptr;
     if (const int rc = prepare_comp(h, P, &comp)) return rc;
     a.clk = h->clk;
@@ -669,15 +666,14 @@ int enqueue_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaE
     a.cfl = o->cfl;
     a.n_disc = o->n_disc;
     a.copy_wait = h->copy_wait;
-    const int shape0 = shape_index(P, 0), shape1 = shape_index(P, 1);
+    const int map = shape_index(P, tiling.shape);
     if (ev) SB_TRY(cudaEventRecord(ev[0], h->stream));
     for (int s = 0; s < nsteps; s++) {
         double* U = h->buf[h->cur];
         double* W = h->buf[1 - h->cur];
-        const CUtensorMap* tmU = h->tma_ok[shape0] ? h->tmap + kNumShapes * h->cur + shape0 : nullptr;
-        const CUtensorMap* tmW = h->tma_ok[shape1] ? h->tmap + kNumShapes * (1 - h->cur) + shape1 : nullptr;
+        const CUtensorMap* tmU = h->tma_ok[map] ? h->tmap + kNumShapes * h->cur + map : nullptr;
+        const CUtensorMap* tmW = h->tma_ok[map] ? h->tmap + kNumShapes * (1 - h->cur) + map : nullptr;
         if (o->scheme == 2) {
-            a.g.lz = lz0;
             a.Uin = U;
             a.tm_in = tmU;
             a.Ubase = nullptr;
@@ -686,7 +682,6 @@ int enqueue_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaE
             a.comp = nullptr;
             SB_TRY(launch_stage(a, P, o->n_state, o->order, 0, h->stream));
             if (ev) SB_TRY(cudaEventRecord(ev[2 * s + 1], h->stream));
-            a.g.lz = lz1;
             a.Uin = W;
             a.tm_in = tmW;
             a.Ubase = U;
@@ -696,7 +691,6 @@ int enqueue_steps(setb_handle* h, int32_t nsteps, const setb_step_opts* o, cudaE
             SB_TRY(launch_stage(a, P, o->n_state, o->order, 1, h->stream));
             if (ev) SB_TRY(cudaEventRecord(ev[2 * s + 2], h->stream));
         } else {
-            a.g.lz = lz0;
             a.Uin = U;
             a.tm_in = tmU;
             a.Ubase = nullptr;
@@ -897,7 +891,6 @@ int32_t setb_init_slab(setb_handle** h, const setb_cart_desc* d, int32_t k0, int
     rc = create_impl(h, d, &g);
     if (rc) return rc;
     setb_handle* s = *h;
-    s->g.lz = choose_lz(s->g, s->sm_count, 0, 0);
     clock_reset(s, 0.0);
     rc = upload_cellpar(s, cell_par);
     if (!rc) rc = upload_clock(s);
@@ -934,17 +927,19 @@ int32_t setb_slab_stage(setb_handle* h, int32_t stage, const setb_step_opts* o) 
                                      cudaMemcpyDeviceToDevice, h->stream));
     float* comp = nullptr;
     if ((rc = prepare_comp(h, P, &comp))) return rc;
-    const int shape = shape_index(P, kind);
+    const Tiling tiling = choose_tiling(g, h->sm_count, P);
+    const int map = shape_index(P, tiling.shape);
     StageArgs a{};
     a.g = g;
-    a.g.lz = choose_lz(g, h->sm_count, P, kind);
+    a.g.lz = tiling.lz;
+    a.shape = tiling.shape;
     a.clk = h->clk;
     a.st = h->st;
     a.cfl = o->cfl;
     a.n_disc = o->n_disc;
     a.copy_wait = h->copy_wait;
     a.Uin = X;
-    a.tm_in = h->tma_ok[shape] ? h->tmap + kNumShapes * in + shape : nullptr;
+    a.tm_in = h->tma_ok[map] ? h->tmap + kNumShapes * in + map : nullptr;
     if (stage == 1) {
         a.Ubase = nullptr;
         a.Uout = W;

@@ -122,7 +122,7 @@ extern "C" int32_t setb_step_noalloc(const setb_cart_desc* d, const setb_step_op
     a.g.v_src = d->v_src;
     a.g.p_over_rho_src = d->p_over_rho_src;
     a.g.r_floor = d->r_floor;
-    a.g.lz = choose_lz(a.g, sms, 0, 0);   // the handle path's z chunking (same tiles, same faces)
+    a.g.lz = choose_tiling(a.g, sms, 0).lz;   // the handle path's z chunking (same tiles, same faces)
     a.clk = clk;
     a.st = st;
     a.cfl = o->cfl;

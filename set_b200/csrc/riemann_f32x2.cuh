@@ -56,11 +56,18 @@ __device__ __forceinline__ void reconstruct_f32x2(const float* qLL, const float*
     if (q2[4] < 0.0f) q2[4] = qR[4];
 }
 
+// BN_FIRST: which product of v.b is rounded before it is summed.  The single-solve kernel and the batch
+// kernel have always differed in this (the compiler's choice once), and FP32 rounding grows over
+// hundreds of steps, so each keeps its own order and reproduces its earlier results bit for bit.
+template <bool BN_FIRST>
+__device__ __forceinline__ float star_vb(float bn, float SM, float b2, float v2, float b3, float v3) {
+    return fmaf(b3, v3, BN_FIRST ? fmaf(b2, v2, __fmul_rn(bn, SM)) : fmaf(bn, SM, __fmul_rn(b2, v2)));
+}
 // Face-frame states q = (rho, vn, vt1, vt2, p, Bn, Bt1, Bt2), B in stored units; F in the same
 // order (B fluxes in stored units); SL, SR, SM as chlld's dsl, dsp, dsc.  Returns kFlagWave when
 // no wave-fan region matched and kFlagStar when the selected state has rho <= 0 or p <= 0 or
 // a flux is not finite (the caller then recomputes the face in FP64).
-template <int NSTATE>
+template <int NSTATE, bool BN_FIRST>
 __device__ __forceinline__ int riemann_f32x2(const float* q1, const float* q2, float* F, float& SLo, float& SRo,
                                              float& SMo) {
     static_assert(NSTATE == 2 || NSTATE == 3, "HLLC or HLLD");
@@ -209,11 +216,11 @@ __device__ __forceinline__ int riemann_f32x2(const float* q1, const float* q2, f
         const float sums = pick(sum, right), isms = pick(ism, right);
         const float rzz = pick(rz, right), S1 = right ? SR : SL, S2 = right ? SZR : SZL;
         const float v2s = pick(vz2, right), v3s = pick(vz3, right), b2z = pick(bz2, right), b3z = pick(bz3, right);
-        const float sbvS = NSTATE == 2 ? sbvz : (bn * SM + b2z * v2s) + b3z * v3s;
+        const float sbvS = NSTATE == 2 ? sbvz : star_vb<BN_FIRST>(bn, SM, b2z, v2s, b3z, v3s);
         const float ez = e * sums + (((ptz * SM - pts * uu) + bn * (sbv - sbvS)) * isms);
         float ezz = ez;
         if (NSTATE == 3 && use2) {
-            const float sbzz = (bn * SM + bzz2 * vzz2) + bzz3 * vzz3;
+            const float sbzz = star_vb<BN_FIRST>(bn, SM, bzz2, vzz2, bzz3, vzz3);
             ezz = right ? ez + pick(rzs, true) * sbn * (sbvS - sbzz) : ez - pick(rzs, false) * sbn * (sbvS - sbzz);
         }
         const F2 uz23 = splat(rzz) * mk(v2s, v3s), uzz23 = splat(rzz) * mk(vzz2, vzz3);

@@ -16,16 +16,20 @@ namespace sb {
 // of 128 registers and the smallest halo (1.43 cells staged per cell; 384^3, stage 1 / 2: 4.82 /
 // 5.58 ms against 5.32 / 6.12 with 11 rows and 12 warps).  A second staged box would fit, but leaves
 // 18 KB of L1 for the second stage's loads: 6.32 against 5.58 ms.
+// The mixed form's second shape, 7 rows in each of two CTAs per SM, is for grids whose rows it pads
+// less (choose_tiling).
 constexpr int kTileX = 32;
 struct TileShape {
     int ty, threads, ctas_per_sm;
+    double interval;   // time of one interval of the march on a full SM, relative to the form's first shape
 };
-SB_HD constexpr TileShape tile_shape(int precision, int kind) {
-    (void)kind;
-    return precision == 1 ? TileShape{15, 512, 1} : TileShape{11, 384, 1};
+SB_HD constexpr int num_shapes(int precision) { return precision == 1 ? 2 : 1; }
+SB_HD constexpr TileShape tile_shape(int precision, int shape) {
+    return precision != 1 ? TileShape{11, 384, 1, 1.0}
+                          : (shape == 0 ? TileShape{15, 512, 1, 1.0} : TileShape{7, 256, 2, 0.97});
 }
-// The tile_shape kind every batch launch uses.
-constexpr int kBatchKind = 1;
+// The shape every batch launch uses.
+constexpr int kBatchShape = 0;
 
 // Clock of one solve, in device memory.  The reference keeps time_step / time_step2 /
 // dev_time_all as device scalars written from the host each step (cuf_kernel.cuf:18-19,
@@ -97,6 +101,8 @@ struct StageArgs {
     const CUtensorMap* tm_in;           // tensor map of Uin (device memory) for the plane
                                         // copies, box (kTileX + 4, ty + 4, 1, 8) of this form's
                                         // tile; null = planes read with plain loads
+    int shape;                          // tile_shape of the launch (single solves)
+    int pad;
     long long copy_wait;                // limit of the first wait for a plane copy, in SM cycles:
                                         // 0 = kCopyWaitCycles, < 0 = one non-blocking check
                                         // (setb_set_copy_wait; tests of the timeout path)
@@ -110,8 +116,11 @@ constexpr long long kCopyWaitCycles = 4000000000ll;
 // (capi.cu): SETB_OK or the status to return.
 int validate_desc(const setb_cart_desc* d);
 int validate_opts(const setb_step_opts* o);
-// z extent of one CTA's march for a grid on sm_count SMs (capi.cu).
-int choose_lz(const GridGeom& g, int sm_count, int precision, int kind);
+// Tile shape and z extent of one CTA's march for a grid on sm_count SMs (capi.cu).
+struct Tiling {
+    int shape, lz;
+};
+Tiling choose_tiling(const GridGeom& g, int sm_count, int precision);
 
 // One launch of the batch kernel: tiles of many solves behind one work-queue counter.
 struct BatchArgs {

@@ -21,6 +21,6 @@ cudaError_t prepare_batch_kernels(int precision) {
     return prepare_batch_form<0>();
 }
 
-int batch_ctas_per_sm(int precision) { return tile_shape(precision, kBatchKind).ctas_per_sm; }
+int batch_ctas_per_sm(int precision) { return tile_shape(precision, kBatchShape).ctas_per_sm; }
 
 }  // namespace sb

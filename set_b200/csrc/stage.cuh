@@ -60,7 +60,7 @@ constexpr int RING = 4;
 // 3 TY + 2 warp jobs of a plane's faces (see run_tile) take three rounds of the CTA's warps
 // (32 x 7 cells: 23 jobs over 8 warps; 32 x 11: 35 jobs over 12 warps).  Threads 0..NC-1 own
 // one cell each in the update.
-template <int P, int SK> struct Tile {   // SK: the launch kind of tile_shape
+template <int P, int SK> struct Tile {   // SK: the shape of tile_shape
     static constexpr int TX = kTileX, TY = tile_shape(P, SK).ty, NT = tile_shape(P, SK).threads;
     static constexpr int MINB = tile_shape(P, SK).ctas_per_sm;
     static constexpr int NC = TX * TY;
@@ -615,7 +615,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int
                 RT SL, SR, SM;
                 if constexpr (P == 1 && NSTATE >= 2) {
                     if (A.n_disc == 0)
-                        fl = riemann_f32x2<NSTATE>(q1, q2, F, SL, SR, SM);
+                        fl = riemann_f32x2<NSTATE, ND != 2>(q1, q2, F, SL, SR, SM);
                     else
                         fl = riemann<RT, NSTATE, false, true, true, false, false>(q1, q2, RT(0), A.n_disc, F, SL, SR, SM);
                 } else if constexpr (P == 0) {
@@ -824,14 +824,14 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int
     __syncthreads();
 }
 
-template <int P, int NSTATE, int ORDER, int KIND, int ND>
-__global__ void __launch_bounds__(Tile<P, KIND>::NT, Tile<P, KIND>::MINB) stage_kernel(const StageArgs A) {
+template <int P, int NSTATE, int ORDER, int KIND, int ND, int SK>
+__global__ void __launch_bounds__(Tile<P, SK>::NT, Tile<P, SK>::MINB) stage_kernel(const StageArgs A) {
     __shared__ __align__(8) unsigned long long bar;
     if (threadIdx.x == 0) mbar_init(&bar);
     __syncthreads();
     unsigned phase = 0;
     bool tma_dead = false;
-    run_tile<P, NSTATE, ORDER, KIND, KIND, ND>(A, blockIdx.x, blockIdx.y, blockIdx.z,
+    run_tile<P, NSTATE, ORDER, KIND, SK, ND>(A, blockIdx.x, blockIdx.y, blockIdx.z,
                                                          gridDim.x * gridDim.y * gridDim.z, &bar, phase, tma_dead);
 }
 
@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(Tile<P, KIND>::NT, Tile<P, KIND>::MINB) stage_
 // one Riemann solver (NSTATE), so the kernel holds one solver body.  The items of one solve are
 // counted by its own clock, so every solve keeps its own lagged dt.
 template <int P, int NSTATE, int ORDER, int KIND>
-__global__ void __launch_bounds__(Tile<P, kBatchKind>::NT, Tile<P, kBatchKind>::MINB) batch_stage_kernel(const BatchArgs B) {
+__global__ void __launch_bounds__(Tile<P, kBatchShape>::NT, Tile<P, kBatchShape>::MINB) batch_stage_kernel(const BatchArgs B) {
     __shared__ __align__(16) StageArgs As;
     __shared__ int4 it;
     __shared__ __align__(8) unsigned long long bar;
@@ -859,17 +859,17 @@ __global__ void __launch_bounds__(Tile<P, kBatchKind>::NT, Tile<P, kBatchKind>::
         if (w.x < 0) break;
         const unsigned long long* src = reinterpret_cast<const unsigned long long*>(B.inst + w.x);
         unsigned long long* dst = reinterpret_cast<unsigned long long*>(&As);
-        for (int q = threadIdx.x; q < WORDS; q += Tile<P, kBatchKind>::NT) dst[q] = src[q];
+        for (int q = threadIdx.x; q < WORDS; q += Tile<P, kBatchShape>::NT) dst[q] = src[q];
         __syncthreads();
-        run_tile<P, NSTATE, ORDER, KIND, kBatchKind, 2>(As, w.y, w.z, w.w, As.total_tiles, &bar,
+        run_tile<P, NSTATE, ORDER, KIND, kBatchShape, 2>(As, w.y, w.z, w.w, As.total_tiles, &bar,
                                                                   phase, tma_dead);
     }
 }
 
-template <int P, int NSTATE, int ORDER, int KIND, int ND>
-cudaError_t launch_nd(const StageArgs& a, cudaStream_t s) {
-    auto kern = stage_kernel<P, NSTATE, ORDER, KIND, ND>;
-    const int smem = Tile<P, KIND>::kSmem;
+template <int P, int NSTATE, int ORDER, int KIND, int ND, int SK>
+cudaError_t launch_shape(const StageArgs& a, cudaStream_t s) {
+    auto kern = stage_kernel<P, NSTATE, ORDER, KIND, ND, SK>;
+    const int smem = Tile<P, SK>::kSmem;
     // The dynamic shared-memory opt-in is a per-device attribute of the kernel: set it once per
     // device ordinal (a bit per device, atomically; two threads that both set it set the same
     // value), and on every launch for ordinals beyond the mask.
@@ -883,11 +883,18 @@ cudaError_t launch_nd(const StageArgs& a, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         attr_set.fetch_or(bit, std::memory_order_release);
     }
-    constexpr int TX = Tile<P, KIND>::TX, TY = Tile<P, KIND>::TY;
+    constexpr int TX = Tile<P, SK>::TX, TY = Tile<P, SK>::TY;
     const int nzu = plane_end(a.g) - plane_begin(a.g);
     dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY, (nzu + a.g.lz - 1) / a.g.lz);
-    kern<<<grid, Tile<P, KIND>::NT, smem, s>>>(a);
+    kern<<<grid, Tile<P, SK>::NT, smem, s>>>(a);
     return cudaGetLastError();
+}
+
+template <int P, int NSTATE, int ORDER, int KIND, int ND>
+cudaError_t launch_nd(const StageArgs& a, cudaStream_t s) {
+    if constexpr (num_shapes(P) > 1)
+        if (a.shape == 1) return launch_shape<P, NSTATE, ORDER, KIND, ND, 1>(a, s);
+    return launch_shape<P, NSTATE, ORDER, KIND, ND, 0>(a, s);
 }
 
 // n_disc selects the wave-speed estimate.  The plain form's HLLC / HLLD for n_disc 0 have a solver
@@ -908,17 +915,17 @@ cudaError_t launch_n(const StageArgs& a, int order, int kind, cudaStream_t s) {
 template <int P, int NSTATE>
 cudaError_t batch_attr() {
     cudaError_t e = cudaFuncSetAttribute(batch_stage_kernel<P, NSTATE, 2, 0>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<P, kBatchKind>::kSmem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<P, kBatchShape>::kSmem);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(batch_stage_kernel<P, NSTATE, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                Tile<P, kBatchKind>::kSmem);
+                                Tile<P, kBatchShape>::kSmem);
 }
 
 template <int P, int NSTATE>
 void launch_batch_n(const BatchArgs& b, int kind, int grid, cudaStream_t s) {
-    constexpr int NT = Tile<P, kBatchKind>::NT;
-    if (kind == 0) batch_stage_kernel<P, NSTATE, 2, 0><<<grid, NT, Tile<P, kBatchKind>::kSmem, s>>>(b);
-    else batch_stage_kernel<P, NSTATE, 2, 1><<<grid, NT, Tile<P, kBatchKind>::kSmem, s>>>(b);
+    constexpr int NT = Tile<P, kBatchShape>::NT;
+    if (kind == 0) batch_stage_kernel<P, NSTATE, 2, 0><<<grid, NT, Tile<P, kBatchShape>::kSmem, s>>>(b);
+    else batch_stage_kernel<P, NSTATE, 2, 1><<<grid, NT, Tile<P, kBatchShape>::kSmem, s>>>(b);
 }
 
 }  // namespace
