@@ -34,9 +34,11 @@ struct setb_handle {
     int cur = 0;                           // buf[cur] holds U^n
     float* comp = nullptr;                 // mixed form: FP32 compensation, 8 * vs floats
     bool comp_clean = false;               // comp holds zeros for the current state
-    DevClock* clk = nullptr;
+    SolveHead* head = nullptr;             // device: clock and counters
+    SolveHead* h_head = nullptr;           // pinned mirror
+    DevClock* clk = nullptr;               // their parts
     DevStatus* st = nullptr;
-    DevClock* h_clk = nullptr;             // pinned mirrors
+    DevClock* h_clk = nullptr;
     DevStatus* h_st = nullptr;
     CUtensorMap* tmap = nullptr;           // device: [buffer 0/1][tile shape, kShapeTy]
     bool tma_ok[3] = {false, false, false};   // per tile shape: maps encoded (else plain loads)
@@ -164,15 +166,13 @@ void clock_reset(setb_handle* h, double time_all) {
 }
 
 int upload_clock(setb_handle* h) {
-    SB_TRY(cudaMemcpyAsync(h->clk, h->h_clk, sizeof(DevClock), cudaMemcpyHostToDevice, h->stream));
-    SB_TRY(cudaMemcpyAsync(h->st, h->h_st, sizeof(DevStatus), cudaMemcpyHostToDevice, h->stream));
+    SB_TRY(cudaMemcpyAsync(h->head, h->h_head, sizeof(SolveHead), cudaMemcpyHostToDevice, h->stream));
     SB_TRY(cudaStreamSynchronize(h->stream));
     return SETB_OK;
 }
 
 int download_clock(setb_handle* h) {
-    SB_TRY(cudaMemcpyAsync(h->h_clk, h->clk, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
-    SB_TRY(cudaMemcpyAsync(h->h_st, h->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->stream));
+    SB_TRY(cudaMemcpyAsync(h->h_head, h->head, sizeof(SolveHead), cudaMemcpyDeviceToHost, h->stream));
     SB_TRY(cudaStreamSynchronize(h->stream));
     return SETB_OK;
 }
@@ -194,12 +194,10 @@ void destroy_impl(setb_handle* h) {
     for (double* b : h->buf)
         if (b) cudaFree(b);
     if (h->comp) cudaFree(h->comp);
-    if (h->clk) cudaFree(h->clk);
-    if (h->st) cudaFree(h->st);
+    if (h->head) cudaFree(h->head);
     if (h->tmap) cudaFree(h->tmap);
     if (h->fl) fl_destroy(h->fl);
-    if (h->h_clk) cudaFreeHost(h->h_clk);
-    if (h->h_st) cudaFreeHost(h->h_st);
+    if (h->h_head) cudaFreeHost(h->h_head);
     if (h->stream) cudaStreamDestroy(h->stream);
     host_pool_release();
     cudaSetDevice(prev);
@@ -219,13 +217,12 @@ int create_impl(setb_handle** out, const setb_cart_desc* d, const GridGeom* geo 
     cudaGetDevice(&h->device);
     h->desc = *d;
     h->g = geo ? *geo : make_geom(d);
-    cudaDeviceProp prop{};
-    if (cudaGetDeviceProperties(&prop, h->device) != cudaSuccess) {
+    if (cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) {
+        cudaGetLastError();
         delete h;
         return SETB_ECUDA;
     }
     host_pool_acquire();   // released by destroy_impl
-    h->sm_count = prop.multiProcessorCount;
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
         h->stream = nullptr;
         destroy_impl(h);
@@ -260,13 +257,16 @@ int create_impl(setb_handle** out, const setb_cart_desc* d, const GridGeom* geo 
             return SETB_ENOMEM;
         }
     }
-    if (cudaMalloc(&h->clk, sizeof(DevClock)) != cudaSuccess || cudaMalloc(&h->st, sizeof(DevStatus)) != cudaSuccess ||
-        cudaMallocHost(&h->h_clk, sizeof(DevClock)) != cudaSuccess ||
-        cudaMallocHost(&h->h_st, sizeof(DevStatus)) != cudaSuccess) {
+    if (cudaMalloc(&h->head, sizeof(SolveHead)) != cudaSuccess ||
+        cudaMallocHost(&h->h_head, sizeof(SolveHead)) != cudaSuccess) {
         cudaGetLastError();
         destroy_impl(h);
         return SETB_ENOMEM;
     }
+    h->clk = &h->head->clk;
+    h->st = &h->head->st;
+    h->h_clk = &h->h_head->clk;
+    h->h_st = &h->h_head->st;
     *out = h;
     return SETB_OK;
 }
@@ -812,8 +812,7 @@ int32_t setb_copy_state(setb_handle* dst, setb_handle* src) {
     SB_TRY(cudaStreamSynchronize(src->stream));
     SB_TRY(cudaMemcpyAsync(dst->buf[dst->cur], src->buf[src->cur], sizeof(double) * 8 * (size_t)src->g.vs,
                            cudaMemcpyDeviceToDevice, dst->stream));
-    SB_TRY(cudaMemcpyAsync(dst->clk, src->clk, sizeof(DevClock), cudaMemcpyDeviceToDevice, dst->stream));
-    SB_TRY(cudaMemcpyAsync(dst->st, src->st, sizeof(DevStatus), cudaMemcpyDeviceToDevice, dst->stream));
+    SB_TRY(cudaMemcpyAsync(dst->head, src->head, sizeof(SolveHead), cudaMemcpyDeviceToDevice, dst->stream));
     dst->comp_clean = false;
     return SETB_OK;
 }

@@ -95,7 +95,9 @@ __device__ __forceinline__ void store_prim(double* P, int64_t c, const double* q
 }
 
 // Primitive state of the first stage of a call (later stages get theirs from the cell kernel).
-__global__ void fl_prim_kernel(int64_t n, const double* __restrict__ U, int64_t vs, double* __restrict__ P) {
+__global__ void fl_prim_kernel(int64_t n, const double* U, int64_t vs, double* P) {
+    allow_successor();
+    wait_for_predecessor();
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
         double u8[8], q[8], ke, me;
 #pragma unroll
@@ -111,7 +113,7 @@ __device__ __forceinline__ void load_prim(const double* P, int64_t c, double* q)
     const double2* p2 = reinterpret_cast<const double2*>(P + 8 * c);
 #pragma unroll
     for (int v = 0; v < NV / 2; v++) {
-        const double2 d = __ldg(p2 + v);
+        const double2 d = p2[v];
         q[2 * v] = d.x;
         q[2 * v + 1] = d.y;
     }
@@ -237,15 +239,18 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
     const int64_t gr = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     double cand = kDtReset;
     unsigned n_recon = 0, n_wave = 0;
-    const int tword = gr < m.n_gran ? m.type[gr] : 0;
+    allow_successor();
+    const int64_t gc = gr < m.n_gran ? gr : m.n_gran - 1;   // geometry: no kernel writes it
+    const int tword = gr < m.n_gran ? __ldg(m.type + gc) : 0;
     const int type = tword & 7;
+    const int4 nb = __ldg(reinterpret_cast<const int4*>(m.nb) + gc);
+    const double2* n2 = reinterpret_cast<const double2*>(m.normal + 4 * gc);
+    const double2 na = __ldg(n2);
+    const double n[3] = {na.x, na.y, __ldg(m.normal + 4 * gc + 2)};
+    const double2* g2 = reinterpret_cast<const double2*>(m.geo + 4 * gc);
+    const double2 ga = __ldg(g2);
+    wait_for_predecessor();
     if (type != 0) {
-        const int4 nb = __ldg(reinterpret_cast<const int4*>(m.nb) + gr);
-        const double2* n2 = reinterpret_cast<const double2*>(m.normal + 4 * gr);
-        const double2 na = __ldg(n2);
-        const double n[3] = {na.x, na.y, __ldg(m.normal + 4 * gr + 2)};
-        const double2* g2 = reinterpret_cast<const double2*>(m.geo + 4 * gr);
-        const double2 ga = __ldg(g2);
         double q1[8], q2[8];
         load_prim(m.prim, nb.x, q1);
         load_prim(m.prim, nb.y, q2);              // a ghost face: cell 1 again
@@ -289,7 +294,7 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
         if (m.powell) {   // :433 as commented there: 0.5 * n.(B1 + B2) * square, B of the chlld states
             const double nbs = dadd(dadd(dmul(n[0], dadd(q1[5], q2[5])), dmul(n[1], dadd(q1[6], q2[6]))),
                                     dmul(n[2], dadd(q1[7], q2[7])));
-            m.divb[gr] = dmul(dmul(0.5 * kSpi4, nbs), __ldg(m.normal + 4 * gr + 3));
+            m.divb[gr] = dmul(dmul(0.5 * kSpi4, nbs), __ldg(m.normal + 4 * gc + 3));
         }
         double F[8], SL, SR;
         bool none;
@@ -305,7 +310,7 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
 #pragma unroll
             for (int v = 0; v < 8; v++) F[v] = 0.0;
         }
-        const double sq = __ldg(m.normal + 4 * gr + 3);
+        const double sq = __ldg(m.normal + 4 * gc + 3);
         double2* f2 = reinterpret_cast<double2*>(m.flux + 8 * gr);
 #pragma unroll
         for (int v = 0; v < 4; v++) f2[v] = make_double2(F[2 * v] * sq, F[2 * v + 1] * sq);
@@ -382,7 +387,7 @@ __device__ __forceinline__ void sum_fluxes(const FlView& m, int64_t c, double* p
 // 2).  Compile-time, so a launch carries only its own code (registers set the occupancy of this
 // gather-bound kernel).
 template <int KIND, int PHYS, bool POWELL>
-__global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, const double* __restrict__ Uin,
+__global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, const double* Uin,
                                                                const double* Ubase, double* Uout, int64_t vs,
                                                                DevClock* clk, DevStatus* st, int finalize, int more) {
     __shared__ unsigned long long cnt[2];
@@ -390,11 +395,13 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, c
     if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
     __syncthreads();
     const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    allow_successor();
+    const int flag = c < m.n_cell ? __ldg(m.cell_flag + c) : 0;
+    wait_for_predecessor();
     const double dt = clk->dt_cur;
     if (c < m.n_cell) {
         double un[8], q[8];
         bool have_q = false;
-        const int flag = m.cell_flag[c];
         if (flag & kFrozen) {
 #pragma unroll
             for (int v = 0; v < 8; v++) un[v] = KIND == 0 ? Uin[v * vs + c] : Ubase[v * vs + c];
@@ -496,7 +503,8 @@ template <int NSTATE, int ORDER, bool WANT_DT>
 void launch_face_o(const FlView& m, bool lax, double cfl, int n_disc, DevClock* clk, DevStatus* st, cudaStream_t s) {
     constexpr bool HAS_FAST = NSTATE >= 2;
     const unsigned grid = (unsigned)((m.n_gran + kFaceThreads - 1) / kFaceThreads);
-#define SB_FACE(F, L) fl_face_kernel<NSTATE, ORDER, WANT_DT, F, L><<<grid, kFaceThreads, 0, s>>>(m, cfl, n_disc, clk, st)
+#define SB_FACE(F, L) \
+    launch_chained(fl_face_kernel<NSTATE, ORDER, WANT_DT, F, L>, grid, kFaceThreads, 0, s, m, cfl, n_disc, clk, st)
     if (HAS_FAST && n_disc == 0) {
         if (lax) SB_FACE(HAS_FAST, true);
         else SB_FACE(HAS_FAST, false);
@@ -711,7 +719,7 @@ cudaError_t fl_launch_stage(const FaceListDev* f, const double* Uin, const doubl
     const FlView& m = f->v;
     if (first) {
         const unsigned pgrid = (unsigned)std::min<int64_t>((m.n_cell + kPrimThreads - 1) / kPrimThreads, 148 * 16);
-        fl_prim_kernel<<<pgrid, kPrimThreads, 0, s>>>(m.n_cell, Uin, vs, m.prim);
+        launch_chained(fl_prim_kernel, pgrid, kPrimThreads, 0, s, m.n_cell, Uin, vs, m.prim);
     }
     switch (o->n_state) {
         case 0: launch_face_n<0>(m, f->physics == 1, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
@@ -720,7 +728,8 @@ cudaError_t fl_launch_stage(const FaceListDev* f, const double* Uin, const doubl
         default: launch_face_n<3>(m, f->physics == 1, o->order, want_dt, o->cfl, o->n_disc, clk, st, s); break;
     }
     const unsigned cgrid = (unsigned)((m.n_cell + kCellThreads - 1) / kCellThreads);
-#define SB_CELL(K, PH, PW) fl_cell_kernel<K, PH, PW><<<cgrid, kCellThreads, 0, s>>>(m, Uin, Ubase, Uout, vs, clk, st, finalize, more)
+#define SB_CELL(K, PH, PW) \
+    launch_chained(fl_cell_kernel<K, PH, PW>, cgrid, kCellThreads, 0, s, m, Uin, Ubase, Uout, vs, clk, st, finalize, more)
     if (f->physics == 1) {
         if (kind == 0) SB_CELL(0, 1, false);
         else SB_CELL(1, 1, false);

@@ -51,6 +51,12 @@ struct DevStatus {
     unsigned long long n_timeout;   // bounded waits on a plane copy that gave up
 };
 
+// Clock and counters of a handle, read and copied together.
+struct SolveHead {
+    DevClock clk;
+    DevStatus st;
+};
+
 // Geometry + boundary data of one Cartesian grid.
 struct GridGeom {
     int nx, ny, nz, lz;             // lz: z extent of one CTA's march
@@ -86,7 +92,7 @@ SB_HD int plane_end(const GridGeom& g) { return g.ke > 0 ? g.ke : g.nz; }
 
 struct StageArgs {
     GridGeom g;
-    const double* __restrict__ Uin;     // state the fluxes are computed from
+    const double* Uin;                  // state the fluxes are computed from
     const double* Ubase;                // stage 2: U^n (may alias Uout: read before written, same thread)
     double* Uout;
     DevClock* clk;
@@ -418,6 +424,33 @@ cudaError_t copy_rows_to_host(void* host, size_t hpitch, const void* dev, size_t
 // Owners of the pinned slots kept between transfers (handles and batches).
 void host_pool_acquire();
 void host_pool_release();
+
+// ---------------------------------------------------------------- back-to-back launches
+// A solve is a chain of dependent kernels.  Launched with programmatic serialization, a kernel's
+// blocks start (and read what no kernel writes) while the last blocks of its predecessor run;
+// wait_for_predecessor() then waits until the predecessor has completed and its writes are visible.
+// Every access to what the chain writes comes after it, and none of them by the read-only path (a
+// kernel's blocks may be resident while its input is still being written).  What it takes out is
+// most of a launch's ramp: 32^3 HLLC, one step per call 72 -> 63 us (with clock and counters copied
+// as one block), axisymmetric 512x256 a step 111 -> 97 us, 64^3 first order 43.6 -> 42.8 us.
+#if defined(__CUDACC__)
+__device__ __forceinline__ void allow_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, P(args)...);
+}
+#endif
 
 // ---------------------------------------------------------------- launch entry points
 // kind 0: Euler step / Heun stage 1 (reduces the dt candidate), kind 1: Heun stage 2.

@@ -102,7 +102,7 @@ __device__ __forceinline__ void fetch_prim64(const StageArgs& A, int i, int j, i
     const long long off = (long long)k * g.ps + (long long)j * g.px + i;
     double U[8];
 #pragma unroll
-    for (int v = 0; v < 8; v++) U[v] = __ldg(A.Uin + v * g.vs + off);
+    for (int v = 0; v < 8; v++) U[v] = __ldcg(A.Uin + v * g.vs + off);   // not by the read-only path: launch_chained
     if constexpr (EXACT) {
         prim_from_cons_guarded<SB>(U, q);
     } else {
@@ -292,7 +292,7 @@ __device__ __forceinline__ void fetch_prim64_f(const FetchArgs& f, int i, int j,
     const long long off = (long long)k * f.ps + (long long)j * f.px + i;
     double U[8];
 #pragma unroll
-    for (int v = 0; v < 8; v++) U[v] = __ldg(f.Uin + v * f.vs + off);
+    for (int v = 0; v < 8; v++) U[v] = __ldcg(f.Uin + v * f.vs + off);
     double ke, me;
     prim_from_cons(U, q, ke, me);
 }
@@ -829,6 +829,8 @@ __global__ void __launch_bounds__(Tile<P, SK>::NT, Tile<P, SK>::MINB) stage_kern
     __shared__ __align__(8) unsigned long long bar;
     if (threadIdx.x == 0) mbar_init(&bar);
     __syncthreads();
+    allow_successor();
+    wait_for_predecessor();
     unsigned phase = 0;
     bool tma_dead = false;
     run_tile<P, NSTATE, ORDER, KIND, SK, ND>(A, blockIdx.x, blockIdx.y, blockIdx.z,
@@ -886,8 +888,7 @@ cudaError_t launch_shape(const StageArgs& a, cudaStream_t s) {
     constexpr int TX = Tile<P, SK>::TX, TY = Tile<P, SK>::TY;
     const int nzu = plane_end(a.g) - plane_begin(a.g);
     dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY, (nzu + a.g.lz - 1) / a.g.lz);
-    kern<<<grid, Tile<P, SK>::NT, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(kern, grid, Tile<P, SK>::NT, smem, s, a);
 }
 
 template <int P, int NSTATE, int ORDER, int KIND, int ND>
