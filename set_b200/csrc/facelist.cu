@@ -71,7 +71,7 @@ struct FaceListDev {
 
 namespace {
 
-constexpr int kFaceThreads = 128, kCellThreads = 256, kPrimThreads = 256;
+constexpr int kFaceThreads = 64, kCellThreads = 256, kPrimThreads = 256;
 constexpr int kInner = 6;     // face type: a type-2 face with a second neighbour
 constexpr int kLaxFace = 8;   // face-type bit: the reference's Lax flux on near-axis faces
 constexpr int kFrozen = 1, kSource = 2;   // cell flags: not updated; inside the source sphere
@@ -218,24 +218,83 @@ __device__ __forceinline__ int axisym_update(const double* Uin, const double* Ub
     return rc;
 }
 
+// The primitive rows of a warp's 32 faces in shared memory: 64-byte rows of the two near cells 80 bytes
+// apart, 48-byte rows (rho, u, v, w, p and one more) of the two far ones 48 apart, so eight lanes
+// reading 16 bytes of their own rows hit different banks.  Every member is called by the whole warp.
+struct FaceRows {
+    static constexpr int kNear1 = 0, kNear2 = 32 * 80, kFar1 = 2 * 32 * 80, kFar2 = kFar1 + 32 * 48;
+    static constexpr int kBytes = kFar2 + 32 * 48;
+    unsigned char* base;
+    int lane;
+    __device__ __forceinline__ explicit FaceRows(unsigned char* b) : base(b), lane(threadIdx.x & 31) {}
+    template <int NV> static __device__ __forceinline__ constexpr int pitch() { return NV == 8 ? 80 : 48; }
+    // Starts the copies of cell `c` of every lane (c < 0: none), NV components each, four lanes a row.
+    template <int NV> __device__ __forceinline__ void fetch(int at, const double* prim, int c) const {
+        const int q = lane & 3;
+#pragma unroll
+        for (int r = 0; r < 32; r += 8) {
+            const int f = r + (lane >> 2);
+            const int64_t cell = __shfl_sync(0xffffffffu, c, f);
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(base + at + pitch<NV>() * f + 16 * q);
+            if (cell >= 0 && 2 * q < NV)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(prim + 8 * cell + 2 * q)
+                             : "memory");
+        }
+    }
+    __device__ __forceinline__ void arrived() const {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+    }
+    template <int NV> __device__ __forceinline__ void own(int at, double* q) const {
+        const double2* p = reinterpret_cast<const double2*>(base + at + pitch<NV>() * lane);
+#pragma unroll
+        for (int v = 0; v < NV / 2; v++) {
+            const double2 d = p[v];
+            q[2 * v] = d.x;
+            q[2 * v + 1] = d.y;
+        }
+    }
+    // Flux rows of the warp's faces (lane's face gr), of those with `keep`.
+    __device__ __forceinline__ void store_flux(double* flux, int64_t gr, const double* F, bool keep) const {
+        const unsigned mask = __ballot_sync(0xffffffffu, keep);   // also: every lane has read its rows
+        double2* own = reinterpret_cast<double2*>(base + kNear1 + 80 * lane);
+#pragma unroll
+        for (int v = 0; v < 4; v++) own[v] = make_double2(F[2 * v], F[2 * v + 1]);
+        __syncwarp();
+        const int q = lane & 3;
+        double2* out = reinterpret_cast<double2*>(flux) + 4 * (gr - lane) + q;
+#pragma unroll
+        for (int r = 0; r < 32; r += 8) {
+            const int f = r + (lane >> 2);
+            if (mask >> f & 1u) out[4 * f] = *reinterpret_cast<const double2*>(base + kNear1 + 80 * f + 16 * q);
+        }
+    }
+};
+
 // One face per thread, cuf_solvers.cuf:243-440 (face speed 0).  Bound by the latency of its gathers
 // and of dependent FP64 operations at 16 warps per SM (128 registers, no spills).  A face's four
 // cells are one 16-byte index load; the solver is the Cartesian path's (riemann_fp64.cuh) on any
 // tangents.  With the cell kernel below, a stage on a 96x80x64 box took 0.235 / 0.225 ms with the
 // library-division solver on the reference's field-aligned basis, a primitive pass before every
-// stage and three index arrays, and 0.169 / 0.167 ms so.
+// stage and three index arrays, 0.169 / 0.167 ms with each thread reading its own rows, and 0.138 /
+// 0.144 ms so.
 // The distance-weighted face value of cell 1, linear(-dff1, q11, -df1, q1, df2, q2) at 0
 // (Solvers.f90:141-150), is q1 + minmod((q1 - q11) df1/(dff1 - df1), (q2 - q1) df1/(df1 + df2)): the
 // weights are geometry, formed at set-up (geo = df1, df1/(df1 + df2), df1/(dff1 - df1),
 // df2/(dff2 - df2); the second weight of side 2 is one minus that of side 1).
+// The rows pass through shared memory, four lanes a row on the way in (cp.async) and out, as in
+// sum_fluxes: a warp has all its 128 rows in flight at once, and the kernel was bound by the L1's
+// throughput (70 %) when each thread read its own rows (96^3: 158 us, so 150 us; blocks of two warps instead of four, 148 us).
 // FAST: n_disc is 0 (HLLC / HLLD by the FP64 solvers).  LAX: the grid may have Lax faces (physics 1).
 template <int NSTATE, int ORDER, bool WANT_DT, bool FAST, bool LAX>
-__global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m, double cfl, int n_disc,
+__global__ void __launch_bounds__(kFaceThreads, 8) fl_face_kernel(const FlView m, double cfl, int n_disc,
                                                                DevClock* clk, DevStatus* st) {
+    __shared__ __align__(16) unsigned char rows[kFaceThreads / 32][FaceRows::kBytes];
     __shared__ double red[kFaceThreads / 32];
     __shared__ unsigned long long cnt[2];
     if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
     __syncthreads();
+    const FaceRows fr(rows[threadIdx.x >> 5]);
     const int64_t gr = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     double cand = kDtReset;
     unsigned n_recon = 0, n_wave = 0;
@@ -250,10 +309,18 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
     const double2* g2 = reinterpret_cast<const double2*>(m.geo + 4 * gc);
     const double2 ga = __ldg(g2);
     wait_for_predecessor();
+    fr.fetch<8>(FaceRows::kNear1, m.prim, nb.x);
+    fr.fetch<8>(FaceRows::kNear2, m.prim, nb.y);   // a ghost face: cell 1 again
+    if (ORDER == 2) {
+        fr.fetch<6>(FaceRows::kFar1, m.prim, nb.z);
+        fr.fetch<6>(FaceRows::kFar2, m.prim, nb.w);
+    }
+    fr.arrived();
+    double F[8] = {};
     if (type != 0) {
         double q1[8], q2[8];
-        load_prim(m.prim, nb.x, q1);
-        load_prim(m.prim, nb.y, q2);              // a ghost face: cell 1 again
+        fr.own<8>(FaceRows::kNear1, q1);
+        fr.own<8>(FaceRows::kNear2, q2);
         if (type == 4) {                          // :318-324 outer boundary
             if (q2[1] > -0.1) q2[1] = -0.1;
         } else if (type == 5) {                   // :325-329 axis
@@ -265,8 +332,8 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
         } else if (ORDER == 2 && nb.z >= 0) {     // :358-412
             const double2 gb = __ldg(g2 + 1);
             double q11[6], q22[6];
-            load_prim<6>(m.prim, nb.z, q11);
-            load_prim<6>(m.prim, nb.w, q22);
+            fr.own<6>(FaceRows::kFar1, q11);
+            fr.own<6>(FaceRows::kFar2, q22);
             const double b1 = ga.y, b2 = 1.0 - ga.y;
             double t1[5], t2[5];
 #pragma unroll
@@ -296,7 +363,7 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
                                     dmul(n[2], dadd(q1[7], q2[7])));
             m.divb[gr] = dmul(dmul(0.5 * kSpi4, nbs), __ldg(m.normal + 4 * gc + 3));
         }
-        double F[8], SL, SR;
+        double SL, SR;
         bool none;
         auto reload = [&](double* m3) {
             asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(m3[0]), "=d"(m3[1]) : "l"(n2));
@@ -311,12 +378,12 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
             for (int v = 0; v < 8; v++) F[v] = 0.0;
         }
         const double sq = __ldg(m.normal + 4 * gc + 3);
-        double2* f2 = reinterpret_cast<double2*>(m.flux + 8 * gr);
 #pragma unroll
-        for (int v = 0; v < 4; v++) f2[v] = make_double2(F[2 * v] * sq, F[2 * v + 1] * sq);
+        for (int v = 0; v < 8; v++) F[v] *= sq;
         // compare-and-select min / max (the library fmin / fmax of doubles are far longer sequences)
         if (WANT_DT) cand = sb_min(kDtFaceCap, cfl * ga.x * rs_rcp(sb_max(fabs(SL), fabs(SR))));
     }
+    fr.store_flux(m.flux, gr, F, type != 0);   // a skipped face keeps its flux
     if (n_recon) atomicAdd(&cnt[0], (unsigned long long)n_recon);
     if (n_wave) atomicAdd(&cnt[1], (unsigned long long)n_wave);
     if (WANT_DT) {
@@ -337,11 +404,17 @@ __global__ void __launch_bounds__(kFaceThreads, 4) fl_face_kernel(const FlView m
     }
 }
 
-// Owner-signed sum of a cell's face fluxes (:691-703), in the order of its face list.  All gathers of
-// three faces are in flight together; a missing face reads the zero row.
+// Owner-signed sums of the face fluxes of a warp's 32 cells (:691-703), each in the order of its face
+// list: lane's cell in pot (and the div-B sum in sks).  Four lanes read one 64-byte flux row together
+// (a thread reading its own rows 16 bytes at a time touches 32 rows an instruction and is bound by
+// the L1's throughput: 96^3 cell update 98 us, so 79 us), eight rows an instruction, twelve
+// instructions in flight; the sums pass through shared memory (`tile`, 32 x 10 doubles of the warp) to
+// the lane that owns the cell.  A missing face reads the zero row.  All lanes take part.
 template <bool POWELL>
-__device__ __forceinline__ void sum_fluxes(const FlView& m, int64_t c, double* pot, double& sks) {
-    const int2* j2 = reinterpret_cast<const int2*>(m.cell_gran + 6 * c);
+__device__ __forceinline__ void sum_fluxes(const FlView& m, int64_t c, double* tile, double* pot, double& sks) {
+    const int lane = threadIdx.x & 31, q = lane & 3, quad = lane >> 2;
+    const int64_t cc = min(c, m.n_cell - 1);
+    const int2* j2 = reinterpret_cast<const int2*>(m.cell_gran + 6 * cc);
     int j[6];
 #pragma unroll
     for (int f = 0; f < 3; f++) {
@@ -349,32 +422,47 @@ __device__ __forceinline__ void sum_fluxes(const FlView& m, int64_t c, double* p
         j[2 * f] = p.x;
         j[2 * f + 1] = p.y;
     }
-    sks = 0.0;
+    const double2* flux = reinterpret_cast<const double2*>(m.flux) + q;
 #pragma unroll
-    for (int v = 0; v < 8; v++) pot[v] = 0.0;
+    for (int h = 0; h < 4; h += 2) {   // cells 8 h + quad, 8 (h + 1) + quad of the warp
+        double2 d[2][6];
+        int jc[2][6];
 #pragma unroll
-    for (int g = 0; g < 6; g += 3) {
-        double2 d[3][4];
-        double db[3];
+        for (int i = 0; i < 2; i++) {
 #pragma unroll
-        for (int f = 0; f < 3; f++) {
-            const int a = abs(j[g + f]);
-            const int64_t row = a ? a - 1 : m.n_gran;
-            const double2* f2 = reinterpret_cast<const double2*>(m.flux + 8 * row);
-#pragma unroll
-            for (int v = 0; v < 4; v++) d[f][v] = f2[v];
-            if (POWELL) db[f] = m.divb[row];
-        }
-#pragma unroll
-        for (int f = 0; f < 3; f++) {
-            const double s = j[g + f] < 0 ? -1.0 : 1.0;
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                pot[2 * v] = fma(s, d[f][v].x, pot[2 * v]);
-                pot[2 * v + 1] = fma(s, d[f][v].y, pot[2 * v + 1]);
+            for (int f = 0; f < 6; f++) {
+                const int x = __shfl_sync(0xffffffffu, j[f], 8 * (h + i) + quad);
+                jc[i][f] = x;
+                d[i][f] = flux[4 * (x ? (int64_t)abs(x) - 1 : m.n_gran)];
             }
-            if (POWELL) sks = fma(s, db[f], sks);
         }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int f = 0; f < 6; f++) {
+                const double s = jc[i][f] < 0 ? -1.0 : 1.0;
+                t.x = fma(s, d[i][f].x, t.x);
+                t.y = fma(s, d[i][f].y, t.y);
+            }
+            *reinterpret_cast<double2*>(tile + 10 * (8 * (h + i) + quad) + 2 * q) = t;
+        }
+    }
+    sks = 0.0;
+    if (POWELL) {
+#pragma unroll
+        for (int f = 0; f < 6; f++) {
+            const double db = m.divb[j[f] ? (int64_t)abs(j[f]) - 1 : m.n_gran];
+            sks = j[f] < 0 ? sks - db : sks + db;
+        }
+    }
+    __syncwarp();
+    const double2* own = reinterpret_cast<const double2*>(tile + 10 * lane);
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const double2 t = own[v];
+        pot[2 * v] = t.x;
+        pot[2 * v + 1] = t.y;
     }
 }
 
@@ -390,6 +478,7 @@ template <int KIND, int PHYS, bool POWELL>
 __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, const double* Uin,
                                                                const double* Ubase, double* Uout, int64_t vs,
                                                                DevClock* clk, DevStatus* st, int finalize, int more) {
+    __shared__ __align__(16) double tiles[kCellThreads / 32][320];
     __shared__ unsigned long long cnt[2];
     __shared__ bool last;
     if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
@@ -399,6 +488,8 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, c
     const int flag = c < m.n_cell ? __ldg(m.cell_flag + c) : 0;
     wait_for_predecessor();
     const double dt = clk->dt_cur;
+    double pot[8], sks;
+    sum_fluxes<POWELL>(m, c, tiles[threadIdx.x >> 5], pot, sks);
     if (c < m.n_cell) {
         double un[8], q[8];
         bool have_q = false;
@@ -410,8 +501,6 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, c
             source_state(m.src, x, y, z, dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z)), q);
             cons_from_prim_exact(q, un);
         } else if (PHYS == 1) {
-            double pot[8], sks;
-            sum_fluxes<false>(m, c, pot, sks);
             load_prim(m.prim, c, q);
             const int rc = axisym_update<KIND>(Uin, Ubase, vs, c, q, pot, m.inv_volume[c], m.cell_center[3 * c],
                                                m.cell_center[3 * c + 1], m.hatom + 8 * c, dt, un);
@@ -422,8 +511,6 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, c
                 atomicAdd(&cnt[1], 1ull);
             }
         } else {
-            double pot[8], sks;
-            sum_fluxes<POWELL>(m, c, pot, sks);
             if (POWELL) {
                 // div-B sources inside the flux sum (cuf_solvers.cuf:529-533 / 729-733, commented
                 // there): momentum + (B/4pi) sks, B + u sks, powell 2 energy + (u.B/4pi) sks, with
