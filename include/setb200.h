@@ -336,7 +336,7 @@ SETB_API int32_t setb_checkpoint_read(const char* path, int32_t n_cell, double* 
 /* ------------------------------------------------------------------ batched solves
  * No counterpart in the reference (one grid per process, cuf_kernel.cuf:351-382).  A batch
  * advances many Cartesian solves of uneven size together: every step is two persistent launches
- * whose CTAs draw 32x8xlz tiles of all active solves from one work queue; each solve keeps its own
+ * whose CTAs draw column tiles of all active solves from one work queue; each solve keeps its own
  * lagged dt and clock, so a solve's results do not depend on what else is in the batch.  Solves
  * are admitted by HBM footprint and can be added or removed between steps (continuous batching).
  * Supported per solve: n_state 2 (HLLC) or 3 (HLLD), order 2, scheme 2, the batch's precision. */

@@ -16,6 +16,7 @@
 //   solve's trajectory and stopping step are the same alone and in any mix.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -189,14 +190,30 @@ int rebuild(setb_batch* b) {
     std::stable_partition(order.begin(), order.end(), [&](const std::pair<long long, int>& o) {
         return b->slots[o.second].opts.n_state == 3;
     });
+    // March length: b->lz at most.  Each tile costs three intervals beside its planes, and the last tiles
+    // of a launch leave SMs idle for about a tile and a half: W (1 + 3 / lz) / slots + 1.5 lz over the W
+    // tile planes of all solves is least at sqrt(2 W / slots).  Where that is below 16 planes the tail
+    // counts and it bounds the marches (5 grids of edges 32-64: 4 planes 0.24 ms a step, 8 0.29, 32
+    // 0.47; 6 of 48-112: 12 planes 1.06 ms, 32 1.34); larger batches hide it behind their large solves
+    // (64 of 48-160: whole columns 13.25 ms, 32 planes 13.6).
+    const TileShape ts = tile_shape(b->precision, kBatchShape);
+    auto columns = [&](const GridGeom& g) {
+        return (double)((g.nx + kTileX - 1) / kTileX) * ((g.ny + ts.ty - 1) / ts.ty);
+    };
+    double planes = 0.0;
+    for (auto& os : order) planes += columns(b->slots[os.second].g) * b->slots[os.second].g.nz;
+    const double lz_tail = std::sqrt(2.0 * planes / (b->sm_count * ts.ctas_per_sm)) + 0.5;
+    const int lz_max = lz_tail < 16.0 ? std::max(1, std::min(b->lz, (int)lz_tail)) : b->lz;
     std::vector<int4> items;
     int n_hlld = 0;
     for (auto& os : order) {
         const int s = os.second;
         Slot& sl = b->slots[s];
         GridGeom g = sl.g;
-        g.lz = std::min(b->lz, g.nz);
-        const int ty = tile_shape(b->precision, kBatchShape).ty;
+        const int lz_cap = std::min(lz_max, g.nz);   // chunks as even as they come
+        const int chunks = (g.nz + lz_cap - 1) / lz_cap;
+        g.lz = (g.nz + chunks - 1) / chunks;
+        const int ty = ts.ty;
         const int ntx = (g.nx + kTileX - 1) / kTileX, nty = (g.ny + ty - 1) / ty, ntz = (g.nz + g.lz - 1) / g.lz;
         for (int bz = 0; bz < ntz; bz++)
             for (int by = 0; by < nty; by++)
@@ -578,8 +595,9 @@ int32_t setb_batch_tune(setb_batch* b, int32_t reps, int32_t* lz_out, int32_t* g
             SB_TRY(cudaMemcpyAsync(&saved[s].second, b->slots[s].st, sizeof(DevStatus), cudaMemcpyDeviceToHost, b->stream));
         }
     SB_TRY(cudaStreamSynchronize(b->stream));
+    // one resident CTA per SM draws the tiles: more CTAs than that (a grid multiple) only queue
     const int lzs[] = {8, 16, 32, 64, 1 << 20};
-    const int gms[] = {1, 2};
+    const int gms[] = {1};
     double best = 1e300;
     int best_lz = b->lz, best_gm = b->grid_mult;
     cudaEvent_t e0, e1;
@@ -604,7 +622,10 @@ int32_t setb_batch_tune(setb_batch* b, int32_t reps, int32_t* lz_out, int32_t* g
             cudaEventSynchronize(e1);
             float ms = 0.f;
             cudaEventElapsedTime(&ms, e0, e1);
-            if (ok && ms / reps < best) {
+            // longer marches only where they win clearly: the first stage alone is timed, and short tiles
+            // balance the second one better (6 grids of edges 48-112: first stage 0.49 ms with 8 and with
+            // 16 planes, a step 1.06 and 1.14 ms)
+            if (ok && ms / reps < 0.98 * best) {
                 best = ms / reps;
                 best_lz = lz;
                 best_gm = gm;
