@@ -125,19 +125,51 @@ int shape_index(int precision, int shape) { return precision == 1 ? 1 + shape : 
 // a small grid has too few columns for the SMs, and shorter marches cost more work but less time
 // (32^3 a stage 56 us at 8 planes, 22 us at one; 64^3 59 us at 8, 49 us at 6).
 // Among shapes, the one whose padded tiles take least time (interval: their relative cost).
+// Tiles that cross the source sphere are slower, by `drag` of an interval for each plane inside it: the
+// mixed and delta forms recompute faces there in FP64, every form recovers pressures exactly (96^3
+// with and without a source: plain 125 / 107 us a stage, mixed 173 / 97, delta 233 / 140).  A launch of
+// one wave waits for them; with more waves the SMs that draw them take fewer tiles, where the last
+// wave has room.  With the drag counted, a stage of 64^3 took 62 us (mixed, 84 without) and 69 (delta,
+// 99), of 96^3 133 (173) and 170 (232), plain 96^3 120 (125); long marches that two CTAs share an
+// SM for hide it (mixed 256^3: 1.47 ms in one wave of 7-row tiles).
 Tiling sb::choose_tiling(const GridGeom& g, int sm_count, int precision) {
+    const double drag = precision == 0 ? 0.3 : (precision == 1 ? 0.9 : 0.7);
     const int nz = plane_end(g) - plane_begin(g);   // planes the stage kernels update
+    // cells inside the sphere along each axis through the origin, [first, last] (first > last: none)
+    int first[3], last[3];
+    const int n[3] = {g.nx, g.ny, plane_end(g)};
+    for (int a = 0; a < 3; a++) {
+        const int off = a == 2 ? g.koff : 0, from = a == 2 ? plane_begin(g) : 0;
+        first[a] = n[a];
+        last[a] = from - 1;
+        if (g.r_src > 0.0) {
+            const double lo = (-g.r_src - g.lo[a]) / g.h[a] - 0.5 - off, hi = (g.r_src - g.lo[a]) / g.h[a] - 0.5 - off;
+            first[a] = (int)std::max<double>(from, std::min<double>(n[a], std::ceil(lo)));
+            last[a] = (int)std::min<double>(n[a] - 1, std::max<double>(from - 1, std::floor(hi)));
+        }
+    }
+    const bool source = first[0] <= last[0] && first[1] <= last[1] && first[2] <= last[2];
+    const int zf = first[2] - plane_begin(g), zl = last[2] - plane_begin(g);
     double best = 1e300;
     Tiling t{0, nz};
     for (int shape = 0; shape < num_shapes(precision); shape++) {
         const TileShape ts = tile_shape(precision, shape);
         const long long cols = (long long)((g.nx + kTileX - 1) / kTileX) * ((g.ny + ts.ty - 1) / ts.ty);
         const long long slots = (long long)sm_count * ts.ctas_per_sm;
+        const long long src_cols =
+            source ? (long long)(last[0] / kTileX - first[0] / kTileX + 1) * (last[1] / ts.ty - first[1] / ts.ty + 1) : 0;
         for (int c = 1; c <= nz; c++) {
             const int lz = (nz + c - 1) / c;
             const long long ctas = cols * ((nz + lz - 1) / lz);
             const long long waves = (ctas + slots - 1) / slots;
-            const double cost = (double)waves * (lz + 3) * ts.interval;
+            double cost = (double)waves * (lz + 3);
+            if (source) {
+                const long long slow = src_cols * (zl / lz - zf / lz + 1);
+                const int inside = std::min(lz, zl - zf + 1);
+                const bool filled_in = ts.ctas_per_sm > 1 && 4 * inside < lz;   // by the SM's other CTA
+                if (!filled_in && (waves == 1 || waves * slots - ctas < slow)) cost += drag * inside;
+            }
+            cost *= ts.interval;
             if (cost < best - 1e-9) {
                 best = cost;
                 t = Tiling{shape, lz};
