@@ -10,7 +10,9 @@
 #include <atomic>
 #include <cstring>
 #include <exception>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 
 #include "setb_internal.cuh"
@@ -156,6 +158,28 @@ bool is_direct(const RowCopy& c) {
     return !c.perm && (c.n * c.width < (64u << 10) || c.dpitch > kSlotBytes || !pageable(c.host));
 }
 
+// The copy where no pinned slot can be had: by the driver, renumbered rows through a pageable buffer.
+cudaError_t copy_unstaged(const RowCopy& c, cudaStream_t s) {
+    if (!c.perm)
+        return c.to_device
+                   ? cudaMemcpy2DAsync(c.dev, c.dpitch, c.host, c.hpitch, c.width, c.n, cudaMemcpyHostToDevice, s)
+                   : cudaMemcpy2DAsync(c.host, c.hpitch, c.dev, c.dpitch, c.width, c.n, cudaMemcpyDeviceToHost, s);
+    const size_t per = std::max<size_t>(1, kSlotBytes / c.dpitch);
+    const std::unique_ptr<char[]> buf(new (std::nothrow) char[per * c.dpitch]);
+    if (!buf) return cudaErrorMemoryAllocation;
+    for (size_t r0 = 0; r0 < c.n; r0 += per) {
+        const size_t m = std::min(per, c.n - r0), bytes = c.dpitch * (m - 1) + c.width;
+        char* dev = static_cast<char*>(c.dev) + c.dpitch * r0;
+        if (c.to_device) move_rows(c, buf.get(), r0, m, true);
+        cudaError_t e = c.to_device ? cudaMemcpyAsync(dev, buf.get(), bytes, cudaMemcpyHostToDevice, s)
+                                    : cudaMemcpyAsync(buf.get(), dev, bytes, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return e;
+        if (!c.to_device) move_rows(c, buf.get(), r0, m, false);
+    }
+    return cudaSuccess;
+}
+
 }  // namespace
 
 void host_pool_acquire() {
@@ -210,7 +234,7 @@ cudaError_t copy_rows(const RowCopy* list, int count, cudaStream_t s) {
         if (!slots[2 * pairs] || !slots[2 * pairs + 1]) break;
     }
     if (pairs == 0) {
-        e = cudaErrorMemoryAllocation;
+        for (int k = 0; k < t.n && e == cudaSuccess; k++) e = copy_unstaged(*t.copy[k], s);
     } else {
         std::thread th[kMaxThreads];
         int started = 0;
