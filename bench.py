@@ -42,13 +42,13 @@ BYTES_STAGE1 = 128   # read U^n (8 x f64), write U* (8 x f64)
 BYTES_STAGE2 = 192   # read U*, U^n, write U^n+1
 BYTES_STEP = BYTES_STAGE1 + BYTES_STAGE2
 # DRAM bytes (read + write) per cell of one plain stage-2 launch, from an ncu capture of that
-# kernel at 160^3 (dram__bytes_read.sum 549.3 MB + dram__bytes_write.sum 226.0 MB over 4.096 M
+# kernel at 160^3 (dram__bytes_read.sum 545.4 MB + dram__bytes_write.sum 225.2 MB over 4.096 M
 # cells); traffic grows with the cell count, so the full-size launch's traffic is this figure
 # times its cells.
-TRAFFIC_STAGE2_PER_CELL = 775.4e6 / 160 ** 3
+TRAFFIC_STAGE2_PER_CELL = 770.6e6 / 160 ** 3
 # FP64 pipe thread instructions (DFMA + DMUL + DADD + DSETP) per cell of the same launch, from
-# the same capture's opcode counts (134.52 M warp instructions x 30.94 threads / 4.096 M cells).
-FP64_OPS_STAGE2_PER_CELL = 1016
+# the same capture's opcode counts (105.22 M warp instructions x 31.86 threads / 4.096 M cells).
+FP64_OPS_STAGE2_PER_CELL = 819
 
 
 def peaks():
