@@ -81,16 +81,22 @@ __device__ __forceinline__ void reconstruct_fp64(const double* qLL, const double
     }
 }
 
-// Fast magnetosonic speed, total pressure pt = p + |b|^2/2.  The 1e-300 keeps the seed of the
-// reciprocal square root finite where the discriminant vanishes (gamma p = |b|^2, no tangential
-// field; or p = b = 0).
+// x, or about 1e-200 where x is below that (zero and negative too): one integer maximum of the high
+// word.  It keeps the seed of a reciprocal square root finite where p or the discriminant is zero, and
+// takes a pressure that its recovery rounded below zero (kinetic energy above ~1e9 times the floor)
+// as none, as riemann()'s clamped square roots do.
+__device__ __forceinline__ double at_least_tiny(double x) {
+    return __hiloint2double(max(__double2hiint(x), 0x16687e92), __double2loint(x));
+}
+
+// Fast magnetosonic speed, total pressure pt = p + |b|^2/2.
 __device__ __forceinline__ double fast_speed(const double* q, double& pt) {
     const double bt2 = fma(q[7], q[7], q[6] * q[6]);
     const double b2 = fma(q[5], q[5], bt2);
     const double hp = (0.5 * kGamma) * q[4];
     const double A = fma(0.5, b2, hp), D = fma(-0.5, b2, hp);
-    const double disc = fma(2.0, hp * bt2, fma(D, D, 1e-300));
-    const double S = A + over_sqrt(disc, disc);
+    const double disc = at_least_tiny(fma(2.0, hp * bt2, D * D));
+    const double S = at_least_tiny(A + over_sqrt(disc, disc));
     pt = fma(0.5, b2, q[4]);
     return over_sqrt(S, q[0] * S);
 }
@@ -135,8 +141,9 @@ __device__ __forceinline__ bool hlld_fp64(const double* q1, const double* q2, do
     const double rz1 = rs1 * i1, rz2 = rs2 * i2;                      // star densities
     const double is1 = rs_rsqrt(rz1), is2 = rs_rsqrt(rz2);
     const double abn = sb_abs(bn) > kEpsB ? sb_abs(bn) : 0.0;
-    const double SZ1 = fma(-abn, is1, SM), SZ2 = fma(abn, is2, SM);   // Alfven speeds, :1660-1676
-    const bool right = !(SM > 0.0);
+    // Alfven speeds, :1660-1676; selected, as 0 * is1 is no number where a cold side recedes (rho* = 0)
+    const double SZ1 = abn > 0.0 ? fma(-abn, is1, SM) : SM, SZ2 = abn > 0.0 ? fma(abn, is2, SM) : SM;
+    const bool right = SM <= 0.0;   // a NaN SM (two cold sides that recede) is left: FL where SL > 0
     const double S1 = pick(SL, SR, right), S2 = pick(SZ1, SZ2, right);
     // the selected side: energy, physical flux (:1368-1404)
     const double r = pick(r1, r2, right), u = pick(u1, u2, right), v = pick(v1, v2, right), w = pick(w1, w2, right);
@@ -203,15 +210,21 @@ struct HydroFan {
 __device__ __forceinline__ void hllc_hydro_fan(double r1, double u1, double p1, double r2, double u2, double p2,
                                                HydroFan& f) {
     // c = sqrt(gamma p / rho) = gamma p / sqrt(gamma p rho)
-    const double g1 = fma(kGamma, p1, 1e-300), g2 = fma(kGamma, p2, 1e-300);
+    const double g1 = at_least_tiny(kGamma * p1), g2 = at_least_tiny(kGamma * p2);
     const double c1 = over_sqrt(g1, g1 * r1), c2 = over_sqrt(g2, g2 * r2);
     f.SL = sb_min(u1 - c1, u2 - c2);
     f.SR = sb_max(u1 + c1, u2 + c2);
     const double su1 = f.SL - u1, su2 = f.SR - u2;
     const double rs1 = r1 * su1, rs2 = r2 * su2;
     f.SM = fma(rs2, u2, fma(-rs1, u1, p1 - p2)) * rs_rcp(rs2 - rs1);
+    // Two cold sides that recede have no contact speed.  A face outside their fan reads none: any finite
+    // one on the far side of the outer wave keeps the terms that are multiplied by 0 there finite.
+    if ((__double2hiint(f.SM) & 0x7ff00000) == 0x7ff00000) {
+        if (f.SR < 0.0) f.SM = f.SR - 1.0;
+        else if (f.SL > 0.0 && !(f.SM <= 0.0)) f.SM = f.SL + 1.0;
+    }
     f.ptz = 0.5 * (fma(rs2, f.SM - u2, p2) + fma(rs1, f.SM - u1, p1));
-    f.right = !(f.SM > 0.0) || f.SR < 0.0;
+    f.right = f.SM <= 0.0 || f.SR < 0.0;
     f.r = pick(r1, r2, f.right);
     f.u = pick(u1, u2, f.right);
     f.p = pick(p1, p2, f.right);
