@@ -9,7 +9,7 @@
 // true> in mhd_core.cuh (chlld, SET_Fortran_Cuda_MHD/Solvers.f90:1190-1855, face speed 0, n_disc 0),
 // on states that carry b = B / sqrt(4 pi), with these differences, each exact in real arithmetic:
 //   * fast speeds from cf^2 = (A + sqrt(D^2 + gamma p bt^2)) / rho, A, D = (gamma p +- |b|^2)/2,
-//     bt the tangential field: the discriminant is a sum of squares (no cancellation, no clamp), and
+//     bt the tangential field: the discriminant is a sum of squares (no cancellation; at_least_tiny for p <= 0), and
 //     cf = S / sqrt(rho S) needs no reciprocal of rho: 22 FP64 operations a side instead of 31;
 //   * products the star states, contact speed and total pressure share (rho (S - u)) formed once;
 //   * the wave-fan region from the sign of SM and the selected side's speeds: with ordered speeds
