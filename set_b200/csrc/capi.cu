@@ -40,7 +40,7 @@ struct setb_handle {
     DevStatus* st = nullptr;
     DevClock* h_clk = nullptr;
     DevStatus* h_st = nullptr;
-    CUtensorMap* tmap = nullptr;           // device: [buffer 0/1][tile shape, kShapeTy]
+    CUtensorMap tmap[2 * 3] = {};          // [buffer 0/1][tile shape, kShapeTy]; a launch takes its own as a parameter
     bool tma_ok[3] = {false, false, false};   // per tile shape: maps encoded (else plain loads)
     FaceListDev* fl = nullptr;             // face-list grid (g is then 1-D: nx = N cells)
     int sm_count = 148;
@@ -227,7 +227,6 @@ void destroy_impl(setb_handle* h) {
         if (b) cudaFree(b);
     if (h->comp) cudaFree(h->comp);
     if (h->head) cudaFree(h->head);
-    if (h->tmap) cudaFree(h->tmap);
     if (h->fl) fl_destroy(h->fl);
     if (h->h_head) cudaFreeHost(h->h_head);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -274,19 +273,12 @@ int create_impl(setb_handle** out, const setb_cart_desc* d, const GridGeom* geo 
         }
     }
     {
-        CUtensorMap tm[2 * kNumShapes] = {};
+        static_assert(sizeof(h->tmap) == sizeof(CUtensorMap) * 2 * kNumShapes, "a map per buffer and shape");
         for (int shape = 0; shape < kNumShapes; shape++) {
             h->tma_ok[shape] = true;
             for (int b = 0; b < 2; b++)
-                if (encode_state_tmap(h->g, h->buf[b], kShapeTy[shape], &tm[kNumShapes * b + shape]) != SETB_OK)
+                if (encode_state_tmap(h->g, h->buf[b], kShapeTy[shape], &h->tmap[kNumShapes * b + shape]) != SETB_OK)
                     h->tma_ok[shape] = false;
-        }
-        if (cudaMalloc(&h->tmap, sizeof(tm)) != cudaSuccess ||
-            cudaMemcpyAsync(h->tmap, tm, sizeof(tm), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
-            cudaStreamSynchronize(h->stream) != cudaSuccess) {
-            cudaGetLastError();
-            destroy_impl(h);
-            return SETB_ENOMEM;
         }
     }
     if (cudaMalloc(&h->head, sizeof(SolveHead)) != cudaSuccess ||

@@ -104,9 +104,11 @@ struct StageArgs {
                                         // (Euler / Heun stage 2); null = plain update
     unsigned total_tiles;               // batch: tiles of this solve in the launch
     int n_state;                        // batch: per-solve Riemann solver (2 HLLC, 3 HLLD)
-    const CUtensorMap* tm_in;           // tensor map of Uin (device memory) for the plane
-                                        // copies, box (kTileX + 4, ty + 4, 1, 8) of this form's
-                                        // tile; null = planes read with plain loads
+    const CUtensorMap* tm_in;           // tensor map of Uin for the plane copies, box
+                                        // (kTileX + 4, ty + 4, 1, 8) of this form's tile; null =
+                                        // planes read with plain loads.  Single solves: in host
+                                        // memory, passed to the kernel as a parameter; batches: in
+                                        // device memory
     int shape;                          // tile_shape of the launch (single solves)
     int pad;
     long long copy_wait;                // limit of the first wait for a plane copy, in SM cycles:

@@ -187,6 +187,12 @@ __device__ __forceinline__ void tma_plane(void* dst, const CUtensorMap* tm, int 
         : "memory");
 }
 
+// A tensor map in global memory that the host wrote, possibly where an earlier map lay: the thread that
+// issues the copies acquires it before its first use (the SM's descriptor cache may hold the earlier one).
+__device__ __forceinline__ void acquire_tmap(const CUtensorMap* tm) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(tm) : "memory");
+}
+
 // Cells c0, c0 + step, ... < c1 of a primitive plane with the boundary rules from a staged box
 // (conserved, [v][y][x] with row HX): inflow beyond x = hi, zero-gradient (clamped index, always
 // inside the box) elsewhere.
@@ -409,6 +415,8 @@ __device__ __forceinline__ void update_cell(const StageArgs& A, const CellState<
 // the solve's clock.  Called by the single-solve kernel (one tile per CTA) and by the batch
 // kernel (tiles of many solves drawn from a work queue); every CTA-wide barrier is reached by all
 // threads, and the function ends with one so a CTA may run the next tile immediately.
+// `tm` is the tensor map of a single solve's A.Uin, a kernel parameter; a batch's lies at A.tm_in, acquired
+// by the caller (A.tm_in is null where planes are read with plain loads).
 // `phase` is the parity of the next wait on the staging box's barrier and `tma_dead` is set once a plane copy did not
 // land within both bounded waits (the thread then reads its planes with plain loads); both are
 // per thread and carried across the tiles a CTA runs.
@@ -433,8 +441,8 @@ __device__ __forceinline__ void update_cell(const StageArgs& A, const CellState<
 // the register moves and no axis dispatch; the code still streams: 4 % of stalls are
 // instruction fetch), the solver unchanged.
 template <int P, int NSTATE, int ORDER, int KIND, int SK, int ND>
-__device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int bz, unsigned total_tiles,
-                                         unsigned long long* bar, unsigned& phase, bool& tma_dead) {
+__device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* tm, int bx, int by, int bz,
+                                         unsigned total_tiles, unsigned long long* bar, unsigned& phase, bool& tma_dead) {
     using RG = typename Types<P>::Ring;
     using FT = typename Types<P>::Flux;
     using RT = typename Types<P>::Math;
@@ -479,7 +487,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int
     constexpr unsigned kPlaneBytes = 8u * PLANE * sizeof(double);
     const int kz_last = k1 + 1;
     auto issue_copy = [&](int kk) {
-        tma_plane(stg, A.tm_in, i0 - 2, j0 - 2, min(max(kk, 0), g.nz - 1), kPlaneBytes, bar);
+        tma_plane(stg, ND == 2 ? A.tm_in : tm, i0 - 2, j0 - 2, min(max(kk, 0), g.nz - 1), kPlaneBytes, bar);
     };
     // Converts plane kk for the cells c0, c0 + step, ... < c1 of this thread.
     auto take_plane = [&](int kk, int c0, int step, int c1) {
@@ -825,7 +833,8 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, int bx, int by, int
 }
 
 template <int P, int NSTATE, int ORDER, int KIND, int ND, int SK>
-__global__ void __launch_bounds__(Tile<P, SK>::NT, Tile<P, SK>::MINB) stage_kernel(const StageArgs A) {
+__global__ void __launch_bounds__(Tile<P, SK>::NT, Tile<P, SK>::MINB)
+    stage_kernel(const StageArgs A, const __grid_constant__ CUtensorMap tm) {
     __shared__ __align__(8) unsigned long long bar;
     if (threadIdx.x == 0) mbar_init(&bar);
     __syncthreads();
@@ -833,8 +842,8 @@ __global__ void __launch_bounds__(Tile<P, SK>::NT, Tile<P, SK>::MINB) stage_kern
     wait_for_predecessor();
     unsigned phase = 0;
     bool tma_dead = false;
-    run_tile<P, NSTATE, ORDER, KIND, SK, ND>(A, blockIdx.x, blockIdx.y, blockIdx.z,
-                                                         gridDim.x * gridDim.y * gridDim.z, &bar, phase, tma_dead);
+    run_tile<P, NSTATE, ORDER, KIND, SK, ND>(A, &tm, blockIdx.x, blockIdx.y, blockIdx.z,
+                                             gridDim.x * gridDim.y * gridDim.z, &bar, phase, tma_dead);
 }
 
 // Persistent batch kernel: each CTA takes tiles from the work queue until it is empty; the
@@ -848,7 +857,11 @@ __global__ void __launch_bounds__(Tile<P, kBatchShape>::NT, Tile<P, kBatchShape>
     __shared__ __align__(8) unsigned long long bar;
     constexpr int WORDS = sizeof(StageArgs) / sizeof(unsigned long long);
     static_assert(sizeof(StageArgs) % sizeof(unsigned long long) == 0, "StageArgs must be 8-byte granular");
-    if (threadIdx.x == 0) mbar_init(&bar);
+    __shared__ int acquired;   // the solve whose tensor map this CTA has acquired
+    if (threadIdx.x == 0) {
+        mbar_init(&bar);
+        acquired = -1;
+    }
     unsigned phase = 0;   // the same in every thread
     bool tma_dead = false;
     for (;;) {
@@ -863,8 +876,12 @@ __global__ void __launch_bounds__(Tile<P, kBatchShape>::NT, Tile<P, kBatchShape>
         unsigned long long* dst = reinterpret_cast<unsigned long long*>(&As);
         for (int q = threadIdx.x; q < WORDS; q += Tile<P, kBatchShape>::NT) dst[q] = src[q];
         __syncthreads();
-        run_tile<P, NSTATE, ORDER, KIND, kBatchShape, 2>(As, w.y, w.z, w.w, As.total_tiles, &bar,
-                                                                  phase, tma_dead);
+        if (threadIdx.x == 0 && acquired != w.x) {
+            if (As.tm_in) acquire_tmap(As.tm_in);
+            acquired = w.x;
+        }
+        run_tile<P, NSTATE, ORDER, KIND, kBatchShape, 2>(As, nullptr, w.y, w.z, w.w, As.total_tiles, &bar, phase,
+                                                         tma_dead);
     }
 }
 
@@ -888,7 +905,7 @@ cudaError_t launch_shape(const StageArgs& a, cudaStream_t s) {
     constexpr int TX = Tile<P, SK>::TX, TY = Tile<P, SK>::TY;
     const int nzu = plane_end(a.g) - plane_begin(a.g);
     dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY, (nzu + a.g.lz - 1) / a.g.lz);
-    return launch_chained(kern, grid, Tile<P, SK>::NT, smem, s, a);
+    return launch_chained(kern, grid, Tile<P, SK>::NT, smem, s, a, a.tm_in ? *a.tm_in : CUtensorMap{});
 }
 
 template <int P, int NSTATE, int ORDER, int KIND, int ND>
