@@ -271,15 +271,17 @@ __device__ __forceinline__ bool has_field(const double* q1, const double* q2) {
     return (b << 1) != 0;
 }
 
-// The plain form's face flux for n_disc 0 (HLLC / HLLD).  HLLC takes the field-free path where no
-// lane of the warp has a field.
+// The plain form's face flux for n_disc 0 (HLLC / HLLD).  HLLC takes the field-free path for a face with
+// no field on either side: by the face and not by its warp, as the two paths round differently and a
+// face on the seam of two tiles is computed in both.  A warp pays for both paths only where it has faces
+// of both kinds.
 template <int NSTATE>
 __device__ __forceinline__ bool flux_fp64(const double* q1, const double* q2, double* F, double& SL, double& SR) {
     static_assert(NSTATE == 2 || NSTATE == 3, "HLLC or HLLD");
     if constexpr (NSTATE == 3) {
         return hlld_fp64(q1, q2, F, SL, SR);
     } else {
-        if (!__any_sync(0xffffffffu, has_field(q1, q2))) return hllc_hydro_fp64(q1, q2, F, SL, SR);
+        if (!has_field(q1, q2)) return hllc_hydro_fp64(q1, q2, F, SL, SR);
         double SM;
         const int fl = riemann<double, 2, false, false, true, true>(q1, q2, 0.0, 0, F, SL, SR, SM);
 #pragma unroll
@@ -314,7 +316,7 @@ template <int NSTATE, bool FAST, typename Reload>
 __device__ __forceinline__ bool flux_normal_fp64(const double* n, Reload reload, const double* q1, const double* q2,
                                                  int n_disc, double* F, double& SL, double& SR) {
     if constexpr (NSTATE == 2 && FAST) {
-        if (!__any_sync(__activemask(), has_field(q1, q2))) {
+        if (!has_field(q1, q2)) {   // by the face, as in flux_fp64: its flux is the same in any numbering
             HydroFan f;
             const double u1 = dot3(n, q1[1], q1[2], q1[3]), u2 = dot3(n, q2[1], q2[2], q2[3]);
             hllc_hydro_fan(q1[0], u1, q1[4], q2[0], u2, q2[4], f);
