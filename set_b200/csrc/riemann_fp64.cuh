@@ -81,11 +81,14 @@ __device__ __forceinline__ void reconstruct_fp64(const double* qLL, const double
     }
 }
 
-// x, or about 1e-200 where x is below that (zero and negative too): one integer maximum of the high
-// word.  It keeps the seed of a reciprocal square root finite where p or the discriminant is zero, and
-// takes a pressure that its recovery rounded below zero (kinetic energy above ~1e9 times the floor)
-// as none, as riemann()'s clamped square roots do.
-__device__ __forceinline__ double at_least_tiny(double x) {
+// x, or about 1e-200 where x is below that (zero and negative too).  It keeps the seed of a reciprocal
+// square root finite where p or the discriminant is zero, and takes a pressure that its recovery rounded
+// below zero (kinetic energy above ~1e9 times the floor) as none, as riemann()'s clamped square roots do.
+// A NaN of either sign stays one, so the faces of an invalid state are found.
+__device__ __forceinline__ double at_least_tiny(double x) { return x < 1e-200 ? 1e-200 : x; }
+// The same by one integer maximum of the high word, for an x whose NaN the caller's result shows by
+// another operand: a NaN with its sign bit set counts as negative here.
+__device__ __forceinline__ double at_least_tiny_bits(double x) {
     return __hiloint2double(max(__double2hiint(x), 0x16687e92), __double2loint(x));
 }
 
@@ -95,8 +98,8 @@ __device__ __forceinline__ double fast_speed(const double* q, double& pt) {
     const double b2 = fma(q[5], q[5], bt2);
     const double hp = (0.5 * kGamma) * q[4];
     const double A = fma(0.5, b2, hp), D = fma(-0.5, b2, hp);
-    const double disc = at_least_tiny(fma(2.0, hp * bt2, D * D));
-    const double S = at_least_tiny(A + over_sqrt(disc, disc));
+    const double disc = at_least_tiny_bits(fma(2.0, hp * bt2, D * D));
+    const double S = at_least_tiny(A + over_sqrt(disc, disc));   // A is NaN where p or the field is
     pt = fma(0.5, b2, q[4]);
     return over_sqrt(S, q[0] * S);
 }
