@@ -220,13 +220,19 @@ __device__ __forceinline__ void hllc_hydro_fan(double r1, double u1, double p1, 
     const double su1 = f.SL - u1, su2 = f.SR - u2;
     const double rs1 = r1 * su1, rs2 = r2 * su2;
     f.SM = fma(rs2, u2, fma(-rs1, u1, p1 - p2)) * rs_rcp(rs2 - rs1);
-    // Two cold sides that recede have no contact speed.  A face outside their fan reads none: any finite
-    // one on the far side of the outer wave keeps the terms that are multiplied by 0 there finite.
-    if ((__double2hiint(f.SM) & 0x7ff00000) == 0x7ff00000) {
-        if (f.SR < 0.0) f.SM = f.SR - 1.0;
-        else if (f.SL > 0.0 && !(f.SM <= 0.0)) f.SM = f.SL + 1.0;
-    }
     f.ptz = 0.5 * (fma(rs2, f.SM - u2, p2) + fma(rs1, f.SM - u1, p1));
+    // Two cold sides that recede have no contact speed, nor has a face beside an invalid state.  A face
+    // outside the fan reads none: any finite contact speed on the far side of the outer wave and any
+    // finite star pressure keep the terms that are multiplied by 0 there finite.
+    if ((__double2hiint(f.SM) & 0x7ff00000) == 0x7ff00000) {
+        if (f.SR < 0.0) {
+            f.SM = f.SR - 1.0;
+            f.ptz = 0.0;
+        } else if (f.SL > 0.0 && !(f.SM <= 0.0)) {
+            f.SM = f.SL + 1.0;
+            f.ptz = 0.0;
+        }
+    }
     f.right = f.SM <= 0.0 || f.SR < 0.0;
     f.r = pick(r1, r2, f.right);
     f.u = pick(u1, u2, f.right);

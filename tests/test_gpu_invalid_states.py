@@ -33,7 +33,7 @@ def cells(n_state, u, value):
 
 @pytest.mark.parametrize("value", [np.nan, -np.nan])
 @pytest.mark.parametrize("u", FLOWS)
-@pytest.mark.parametrize("n_state,order", [(3, 1)])
+@pytest.mark.parametrize("n_state,order", [(3, 1), (2, 1)])
 def test_cartesian(n_state, order, u, value):
     inflow, cp = cells(n_state, u, value)
     desc = S.cart_desc(SHAPE, inflow=inflow, r_src=0.0, dt_init=1e-4)
