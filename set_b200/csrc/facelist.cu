@@ -342,14 +342,17 @@ __global__ void __launch_bounds__(kFaceThreads, 8) fl_face_kernel(const FlView m
                 double h;
                 const double m1 = slope((q1[v] - q11[v]) * gb.x, dq * b1, h);
                 t1[v] = fma(h + h, m1, q1[v]);
-                const double m2 = slope(dq * b2, (q22[v] - q2[v]) * gb.y, h);
+                const double m2 = slope((q22[v] - q2[v]) * gb.y, dq * b2, h);
                 t2[v] = fma(-(h + h), m2, q2[v]);
             }
-            if (sb_neg(sum_neg(t1[0], t1[4], t2[0], t2[4]))) {
-                if (sb_neg(t1[0])) t1[0] = q1[0];
-                if (sb_neg(t1[4])) t1[4] = q1[4];
-                if (sb_neg(t2[0])) t2[0] = q2[0];
-                if (sb_neg(t2[4])) t2[4] = q2[4];
+            if (face_values_bad(t1[0], t1[4], t2[0], t2[4])) {
+                fr.own<8>(FaceRows::kNear1, q1);   // type 2 and ghost faces are first order: the cells' own rows
+                fr.own<8>(FaceRows::kNear2, q2);
+#pragma unroll
+                for (int v = 0; v < 5; v++) {
+                    t1[v] = mend_face_value(v, t1[v], q1[v]);
+                    t2[v] = mend_face_value(v, t2[v], q2[v]);
+                }
             }
 #pragma unroll
             for (int v = 0; v < 5; v++) {

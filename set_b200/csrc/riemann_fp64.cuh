@@ -43,20 +43,32 @@ __device__ __forceinline__ double pick(double l, double r, bool right) { return 
 // MUSCL-minmod slope halves: q = t_c +- h m with m the argument of smaller magnitude and h = 1/2, or
 // 0 where the signs differ (one selected word instead of two; minmod() of mhd_core.cuh otherwise).
 // One FP64 compare instead of minmod's 64-bit integer compare: two issue slots fewer, and a slope
-// is used for both of its faces' values where a caller has both.
+// is used for both of its faces' values where a caller has both.  An a that is no
+// number gives b (the far cell's difference comes first); a b that is none stays (face_values_bad).
 __device__ __forceinline__ double slope(double a, double b, double& h) {
     h = (__double2hiint(a) ^ __double2hiint(b)) < 0 ? 0.0 : 0.5;
     return fabs(a) < fabs(b) ? a : b;
 }
-__device__ __forceinline__ double sum_neg(double a, double b, double c, double d) {
-    return __hiloint2double(__double2hiint(a) | __double2hiint(b) | __double2hiint(c) | __double2hiint(d), 0);
+
+// Whether a pair of face states needs its cells' values: a negative density or pressure
+// (cuf_solvers.cuf:394-406), or a neighbour that is no valid state (a cell's pressure is NaN where any of
+// its conserved variables is, so the pressures show it).
+__device__ __forceinline__ bool face_values_bad(double r1, double p1, double r2, double p2) {
+    const unsigned r = max((unsigned)__double2hiint(r1), (unsigned)__double2hiint(r2));
+    const unsigned p = max((unsigned)__double2hiint(p1), (unsigned)__double2hiint(p2));
+    return max(r, p) >= 0x7ff00000u;   // the sign bit, or the exponent of infinities and NaNs
+}
+// Component v (0 density, 4 pressure) of such a state: the cell's value c instead of x.
+__device__ __forceinline__ double mend_face_value(int v, double x, double c) {
+    return (v == 0 || v == 4 ? x >= 0.0 : x == x) ? x : c;
 }
 
 // Face states from the 4-cell stencil (face-frame order; reconstruct() of mhd_core.cuh): second
-// order in rho, v, p with the positivity fallback of cuf_solvers.cuf:394-406, B first order.
-template <int ORDER>
+// order in rho, v, p with the positivity fallback of cuf_solvers.cuf:394-406, B first order.  cell(s, v)
+// gives component v of the left (s = 0) or right cell once more.
+template <int ORDER, typename Cell>
 __device__ __forceinline__ void reconstruct_fp64(const double* qLL, const double* qL, const double* qR,
-                                                 const double* qRR, double* q1, double* q2) {
+                                                 const double* qRR, double* q1, double* q2, Cell cell) {
 #pragma unroll
     for (int v = 0; v < 8; v++) {
         q1[v] = qL[v];
@@ -69,14 +81,15 @@ __device__ __forceinline__ void reconstruct_fp64(const double* qLL, const double
             double h;
             const double m1 = slope(qL[v] - qLL[v], d, h);
             q1[v] = fma(h, m1, qL[v]);
-            const double m2 = slope(d, qRR[v] - qR[v], h);
+            const double m2 = slope(qRR[v] - qR[v], d, h);
             q2[v] = fma(-h, m2, qR[v]);
         }
-        if (sb_neg(sum_neg(q1[0], q1[4], q2[0], q2[4]))) {
-            if (sb_neg(q1[0])) q1[0] = qL[0];
-            if (sb_neg(q1[4])) q1[4] = qL[4];
-            if (sb_neg(q2[0])) q2[0] = qR[0];
-            if (sb_neg(q2[4])) q2[4] = qR[4];
+        if (face_values_bad(q1[0], q1[4], q2[0], q2[4])) {
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                q1[v] = mend_face_value(v, q1[v], cell(0, v));
+                q2[v] = mend_face_value(v, q2[v], cell(1, v));
+            }
         }
     }
 }

@@ -251,7 +251,9 @@ __device__ __forceinline__ void face_states(const RG* pLL, const RG* pL, const R
         qRR[v] = (ORDER == 2 && v < 5) ? (RT)pRR[o] : RT(0);
     }
     if constexpr (P == 1 && ORDER == 2) reconstruct_f32x2(qLL, qL, qR, qRR, q1, q2);
-    else if constexpr (P == 0) reconstruct_fp64<ORDER>(qLL, qL, qR, qRR, q1, q2);
+    else if constexpr (P == 0)
+        reconstruct_fp64<ORDER>(qLL, qL, qR, qRR, q1, q2,
+                                [&](int s, int v) { return (s ? pR : pL)[face_perm<AX>(v) * PLANE]; });
     else reconstruct<RT, ORDER>(qLL, qL, qR, qRR, q1, q2);
 }
 
@@ -573,12 +575,12 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
                     q2[v] = (RT)pR[o];
                     if (ORDER == 2 && v < 5) {
                         const RT c = q2[v];
-                        RT h = RT(0.5), m;
-                        if constexpr (P == 0) m = slope(c - q1[v], (RT)pRR[o] - c, h);
-                        else m = minmod(c - q1[v], (RT)pRR[o] - c);
+                        // minmod() and not slope(): either far cell may be invalid here, this
+                        // face's or the next one's
+                        const RT m = minmod(c - q1[v], (RT)pRR[o] - c);
                         q1[v] = zl[v];
-                        q2[v] = c - h * m;
-                        zl[v] = c + h * m;
+                        q2[v] = c - RT(0.5) * m;
+                        zl[v] = c + RT(0.5) * m;
                         if (v == 0 || v == 4) {
                             if (sb_neg(q2[v])) q2[v] = c;
                             if (sb_neg(zl[v])) zl[v] = c;

@@ -7,6 +7,7 @@ import pytest
 
 import oracle as O
 import set_b200 as S
+from set_b200 import facelist as FL
 from tests.test_gpu_parity import oracle_opts, oracle_problem
 
 pytestmark = pytest.mark.gpu
@@ -33,7 +34,7 @@ def cells(n_state, u, value):
 
 @pytest.mark.parametrize("value", [np.nan, -np.nan])
 @pytest.mark.parametrize("u", FLOWS)
-@pytest.mark.parametrize("n_state,order", [(3, 1), (2, 1)])
+@pytest.mark.parametrize("n_state,order", [(3, 1), (2, 1), (3, 2), (2, 2)])
 def test_cartesian(n_state, order, u, value):
     inflow, cp = cells(n_state, u, value)
     desc = S.cart_desc(SHAPE, inflow=inflow, r_src=0.0, dt_init=1e-4)
@@ -43,4 +44,21 @@ def test_cartesian(n_state, order, u, value):
     _, do = O.run(g, oracle_opts(o), Uo, 1)
     with S.Solver(desc, cell_par=cp) as s:
         s.step(1, o, check=False)
+        compare(s.conserved(), s.status().n_wave_err, Uo, do.n_wave_err)
+
+
+@pytest.mark.parametrize("value", [np.nan, -np.nan])
+@pytest.mark.parametrize("u", FLOWS)
+@pytest.mark.parametrize("n_state,order", [(3, 1), (2, 1), (3, 2), (2, 2)])
+def test_face_list(n_state, order, u, value):
+    _, cp = cells(n_state, u, value)
+    m = FL.box_facelist(SHAPE, permute_seed=4, seed=1, stretch=0.2, sides={"y-": 2, "x-": 2, "x+": 2})
+    at = np.lexsort((m.cell_center[:, 0], m.cell_center[:, 1], m.cell_center[:, 2]))
+    par = FL.fl_params(r_src=0.0, dt_init=1e-4)
+    cpm = np.zeros_like(cp)
+    cpm[at] = cp
+    Uo = O.cellpar_to_cons(cpm, (m.n_cell,)).reshape(8, -1).copy()
+    _, do, _ = O.fl_run(O.facelist(m, par), O.make_opts(n_state, order, 1, 0.4), Uo, 1)
+    with FL.FaceListSolver(m, cpm, par) as s:
+        s.step(1, S.step_opts(n_state=n_state, scheme=1, order=order), check=False)
         compare(s.conserved(), s.status().n_wave_err, Uo, do.n_wave_err)
