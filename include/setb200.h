@@ -357,10 +357,13 @@ SETB_API int32_t setb_batch_check(setb_batch* b, double* rel_change);
 SETB_API int32_t setb_batch_get_conserved(setb_batch* b, int32_t slot, double* U);
 SETB_API int32_t setb_batch_status(setb_batch* b, int32_t slot, setb_diag* out);
 SETB_API int32_t setb_batch_info(setb_batch* b, int64_t* bytes_used, int32_t* active, int32_t* lz, int32_t* grid);
-/* Tiling of the batch launches: z-march length lz and persistent CTAs per SM slot multiplier. */
+/* Tiling of the batch launches: z-march length lz, used as given from here on, and persistent CTAs per
+ * SM slot multiplier.  Without it (or setb_batch_tune) the length follows the members; setb_batch_info
+ * reports the length that runs. */
 SETB_API int32_t setb_batch_set_tiling(setb_batch* b, int32_t lz, int32_t grid_mult);
 /* Autotuner: times `reps` first-stage launches (idempotent on the state) for each candidate
- * tiling on the current membership, keeps the fastest. */
+ * tiling on the current membership, keeps the fastest: the members' own length, of at most the
+ * returned 32 planes, unless a length set as by setb_batch_set_tiling is 2 % faster. */
 SETB_API int32_t setb_batch_tune(setb_batch* b, int32_t reps, int32_t* lz, int32_t* grid_mult, double* ms);
 SETB_API int32_t setb_batch_sync(setb_batch* b);
 SETB_API int32_t setb_batch_destroy(setb_batch* b);

@@ -31,6 +31,7 @@ namespace {
 
 constexpr int kCheckBlocks = 64;     // fixed partial count per solve: deterministic reduction
 constexpr int kMaxGraphSteps = 64;   // steps captured in one graph
+constexpr int kDefaultLz = 32;       // bound of the march length where none is set
 // Device memory a batch keeps from retired solves (the default pool returns it to the driver at every
 // synchronisation, and mapping a slot anew costs milliseconds).
 constexpr unsigned long long kKeepBytes = 4ull << 30;
@@ -123,7 +124,8 @@ struct setb_batch {
     void* h_check_args = nullptr;  // pinned staging for the check kernel arguments
     double* h_check = nullptr;
     // tuning
-    int lz = 32;
+    int lz = kDefaultLz;           // march length: as it is where fixed (set by the caller or the tuner), else a bound
+    bool lz_fixed = false;
     int grid_mult = 1;
     // graph cache
     bool dirty = true;
@@ -179,6 +181,35 @@ void drop_graph(setb_batch* b) {
     b->graph_steps = 0;
 }
 
+// Columns of a grid in the batch's tile shape.
+double tile_columns(const TileShape& ts, const GridGeom& g) {
+    return (double)((g.nx + kTileX - 1) / kTileX) * ((g.ny + ts.ty - 1) / ts.ty);
+}
+
+// March length of the current members, in planes.  A fixed one is taken as it is.  Otherwise b->lz at
+// most: each tile costs three intervals beside its planes, and the last tiles of a launch leave SMs idle
+// for about a tile and a half: W (1 + 3 / lz) / slots + 1.5 lz over the W tile planes of all solves is
+// least at sqrt(2 W / slots).  Where that is below 16 planes the tail counts and it bounds the marches (5
+// grids of edges 32-64: 4 planes 0.24 ms a step, 8 0.29, 32 0.47; 6 of 48-112: 12 planes 1.06 ms, 32
+// 1.34); larger batches hide it behind their large solves (64 of 48-160: whole columns 13.25 ms, 32
+// planes 13.6).
+int march_length(const setb_batch* b) {
+    const TileShape ts = tile_shape(b->precision, kBatchShape);
+    double planes = 0.0;
+    int nz = 0;
+    for (auto& s : b->slots)
+        if (s.active) {
+            planes += tile_columns(ts, s.g) * s.g.nz;
+            nz = std::max(nz, s.g.nz);
+        }
+    int lz = b->lz;
+    if (!b->lz_fixed) {
+        const double lz_tail = std::sqrt(2.0 * planes / (b->sm_count * ts.ctas_per_sm)) + 0.5;
+        if (lz_tail < 16.0) lz = std::max(1, std::min(lz, (int)lz_tail));
+    }
+    return nz ? std::min(lz, nz) : b->lz;
+}
+
 // Rebuilds the per-slot stage arguments and the work list (largest solves first).
 int rebuild(setb_batch* b) {
     const int ms = (int)b->slots.size();
@@ -190,20 +221,8 @@ int rebuild(setb_batch* b) {
     std::stable_partition(order.begin(), order.end(), [&](const std::pair<long long, int>& o) {
         return b->slots[o.second].opts.n_state == 3;
     });
-    // March length: b->lz at most.  Each tile costs three intervals beside its planes, and the last tiles
-    // of a launch leave SMs idle for about a tile and a half: W (1 + 3 / lz) / slots + 1.5 lz over the W
-    // tile planes of all solves is least at sqrt(2 W / slots).  Where that is below 16 planes the tail
-    // counts and it bounds the marches (5 grids of edges 32-64: 4 planes 0.24 ms a step, 8 0.29, 32
-    // 0.47; 6 of 48-112: 12 planes 1.06 ms, 32 1.34); larger batches hide it behind their large solves
-    // (64 of 48-160: whole columns 13.25 ms, 32 planes 13.6).
     const TileShape ts = tile_shape(b->precision, kBatchShape);
-    auto columns = [&](const GridGeom& g) {
-        return (double)((g.nx + kTileX - 1) / kTileX) * ((g.ny + ts.ty - 1) / ts.ty);
-    };
-    double planes = 0.0;
-    for (auto& os : order) planes += columns(b->slots[os.second].g) * b->slots[os.second].g.nz;
-    const double lz_tail = std::sqrt(2.0 * planes / (b->sm_count * ts.ctas_per_sm)) + 0.5;
-    const int lz_max = lz_tail < 16.0 ? std::max(1, std::min(b->lz, (int)lz_tail)) : b->lz;
+    const int lz_max = march_length(b);
     std::vector<int4> items;
     int n_hlld = 0;
     for (auto& os : order) {
@@ -570,7 +589,7 @@ int32_t setb_batch_info(setb_batch* b, int64_t* bytes_used, int32_t* active, int
     for (auto& s : b->slots) n += s.active ? 1 : 0;
     if (bytes_used) *bytes_used = b->used;
     if (active) *active = n;
-    if (lz) *lz = b->lz;
+    if (lz) *lz = march_length(b);
     if (grid) *grid = grid_size(b, b->n_items);
     return SETB_OK;
 }
@@ -578,6 +597,7 @@ int32_t setb_batch_info(setb_batch* b, int64_t* bytes_used, int32_t* active, int
 int32_t setb_batch_set_tiling(setb_batch* b, int32_t lz, int32_t grid_mult) {
     if (!b || lz < 1 || grid_mult < 1 || grid_mult > 8) return SETB_EINVAL;
     b->lz = lz;
+    b->lz_fixed = true;
     b->grid_mult = grid_mult;
     b->dirty = true;
     return SETB_OK;
@@ -596,18 +616,24 @@ int32_t setb_batch_tune(setb_batch* b, int32_t reps, int32_t* lz_out, int32_t* g
         }
     SB_TRY(cudaStreamSynchronize(b->stream));
     // one resident CTA per SM draws the tiles: more CTAs than that (a grid multiple) only queue
-    const int lzs[] = {8, 16, 32, 64, 1 << 20};
+    // 0: the members' own length (march_length), which goes on following them where none beats it
+    const int lzs[] = {0, 8, 16, 32, 64, 1 << 20};
     const int gms[] = {1};
     double best = 1e300;
-    int best_lz = b->lz, best_gm = b->grid_mult;
+    int best_lz = 0, best_gm = b->grid_mult;
+    std::vector<int> timed;   // lengths that run
     cudaEvent_t e0, e1;
     SB_TRY(cudaEventCreate(&e0));
     SB_TRY(cudaEventCreate(&e1));
     for (int lz : lzs)
         for (int gm : gms) {
-            b->lz = lz;
+            b->lz = lz ? lz : kDefaultLz;
+            b->lz_fixed = lz != 0;
             b->grid_mult = gm;
             b->dirty = true;
+            const int runs = march_length(b);
+            if (std::find(timed.begin(), timed.end(), runs) != timed.end()) continue;
+            timed.push_back(runs);
             if (rebuild(b)) continue;
             if (b->n_items == 0) continue;
             auto launch_once = [&]() -> bool {
@@ -633,7 +659,8 @@ int32_t setb_batch_tune(setb_batch* b, int32_t reps, int32_t* lz_out, int32_t* g
         }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    b->lz = best_lz;
+    b->lz = best_lz ? best_lz : kDefaultLz;
+    b->lz_fixed = best_lz != 0;
     b->grid_mult = best_gm;
     b->dirty = true;
     for (size_t s = 0; s < b->slots.size(); s++)
@@ -642,7 +669,7 @@ int32_t setb_batch_tune(setb_batch* b, int32_t reps, int32_t* lz_out, int32_t* g
             SB_TRY(cudaMemcpyAsync(b->slots[s].st, &saved[s].second, sizeof(DevStatus), cudaMemcpyHostToDevice, b->stream));
         }
     SB_TRY(cudaStreamSynchronize(b->stream));
-    if (lz_out) *lz_out = best_lz;
+    if (lz_out) *lz_out = b->lz;
     if (grid_mult_out) *grid_mult_out = best_gm;
     if (ms_out) *ms_out = best;
     return SETB_OK;
