@@ -203,12 +203,12 @@ SETB_API int32_t setb_status(setb_handle* h, setb_diag* out);
 /* No counterpart in the reference (its kernels have no device-side waits).  Sets how long the
  * handle's stage kernels wait for a plane copy (the tensor copy that stages each z plane into
  * shared memory) before they count the wait as run out: cycles > 0 is the limit in SM clock
- * cycles, 0 restores the default (~2 s), cycles < 0 makes every wait a single non-blocking check
- * and checks each tile's first copy right behind its issue (used by tests to drive the error path).  A wait that runs out is reported as SETB_ETIMEOUT by
- * the next call that reads the counters (setb_step with time_all, setb_sync, setb_status); the
- * kernel then gives the copy a second ~2 s wait before it reads the plane, and a copy that never
- * lands switches that thread to plain loads, so the state stays valid.  setb_set_state clears the
- * counters. */
+ * cycles, 0 restores the default (~2 s), cycles < 0 issues each copy right before its wait and
+ * makes the wait a single non-blocking check (used by tests to drive the error path).  A wait that
+ * runs out is reported as SETB_ETIMEOUT by the next call that reads the counters (setb_step with
+ * time_all, setb_sync, setb_status); the kernel then gives the copy a second ~2 s wait before it
+ * reads the plane, and a copy that never lands switches that thread to plain loads, so the state
+ * stays valid.  setb_set_state clears the counters. */
 SETB_API int32_t setb_set_copy_wait(setb_handle* h, int64_t cycles);
 
 /* The CUDA stream the handle launches on (as a void* cudaStream_t). */

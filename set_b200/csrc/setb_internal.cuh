@@ -112,7 +112,8 @@ struct StageArgs {
     int shape;                          // tile_shape of the launch (single solves)
     int pad;
     long long copy_wait;                // limit of the first wait for a plane copy, in SM cycles:
-                                        // 0 = kCopyWaitCycles, < 0 = one non-blocking check
+                                        // 0 = kCopyWaitCycles, < 0 = one non-blocking check of a
+                                        // copy issued right before it
                                         // (setb_set_copy_wait; tests of the timeout path)
 };
 

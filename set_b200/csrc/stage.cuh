@@ -486,6 +486,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
     // next plane is in flight while the faces and the update of an interval run; the last copy
     // issued is plane k1+1.
     const bool use_tma = A.tm_in != nullptr && !tma_dead;
+    const bool late = A.copy_wait < 0;   // each copy issued right before its waits, which run out
     constexpr unsigned kPlaneBytes = 8u * PLANE * sizeof(double);
     const int kz_last = k1 + 1;
     auto issue_copy = [&](int kk) {
@@ -495,6 +496,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
     auto take_plane = [&](int kk, int c0, int step, int c1) {
         RG* slot = ring + ring_slot(kk) * 8 * PLANE;
         if (use_tma && !tma_dead) {
+            if (late && t == 0) issue_copy(kk);
             // A wait that runs out is counted (SETB_ETIMEOUT), then the copy gets a second bounded
             // wait to land before the box is read; a copy that never lands switches this thread to
             // plain loads (and thread 0 stops issuing copies), so no read races a late copy.
@@ -509,15 +511,12 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
         }
         if (!use_tma || tma_dead) load_planes<P, SK, RG>(A, ring, i0, j0, kk, c1, c0, step);
         __syncthreads();
-        if (use_tma && !tma_dead && t == 0 && kk < kz_last) issue_copy(kk + 1);
+        if (use_tma && !tma_dead && !late && t == 0 && kk < kz_last) issue_copy(kk + 1);
     };
     // The first four planes come by plain loads, all in flight together, while the first copy (plane
     // k0+2) runs: the values are the same, and four copies one after the other through the staging
     // box would take four latencies (32^3 a stage: 22 -> 20 us).
-    if (use_tma && t == 0) issue_copy(k0 + 2);
-    // a negative wait limit is one check of the tile's first copy right behind its issue (by the time
-    // the faces are done it has landed)
-    if (use_tma && A.copy_wait < 0 && !mbar_test_wait(bar, phase)) n_tmo++;
+    if (use_tma && !late && t == 0) issue_copy(k0 + 2);
     load_planes<P, SK, RG>(A, ring, i0, j0, k0 - 2, 4 * PLANE, t, NT);
     __syncthreads();
 
