@@ -158,8 +158,9 @@ Tiling sb::choose_tiling(const GridGeom& g, int sm_count, int precision) {
         const long long slots = (long long)sm_count * ts.ctas_per_sm;
         const long long src_cols =
             source ? (long long)(last[0] / kTileX - first[0] / kTileX + 1) * (last[1] / ts.ty - first[1] / ts.ty + 1) : 0;
-        for (int c = 1; c <= nz; c++) {
+        for (int c = 1; c <= nz;) {   // every length that occurs once: about 2 sqrt(nz) of them
             const int lz = (nz + c - 1) / c;
+            c = lz > 1 ? (nz + lz - 2) / (lz - 1) : nz + 1;   // the fewest chunks that are shorter
             const long long ctas = cols * ((nz + lz - 1) / lz);
             const long long waves = (ctas + slots - 1) / slots;
             double cost = (double)waves * (lz + 3);
