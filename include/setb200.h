@@ -339,6 +339,8 @@ SETB_API int32_t setb_checkpoint_read(const char* path, int32_t n_cell, double* 
  * whose CTAs draw column tiles of all active solves from one work queue; each solve keeps its own
  * lagged dt and clock, so a solve's results do not depend on what else is in the batch.  Solves
  * are admitted by HBM footprint and can be added or removed between steps (continuous batching).
+ * A batch keeps up to 4 GiB of its retired solves' memory, within its budget, for new ones until it is
+ * destroyed or another allocation on the device needs it.
  * Supported per solve: n_state 2 (HLLC) or 3 (HLLD), order 2, scheme 2, the batch's precision. */
 typedef struct setb_batch setb_batch;
 

@@ -33,7 +33,9 @@ constexpr int kCheckBlocks = 64;     // fixed partial count per solve: determini
 constexpr int kMaxGraphSteps = 64;   // steps captured in one graph
 constexpr int kDefaultLz = 32;       // bound of the march length where none is set
 // Device memory a batch keeps from retired solves (the default pool returns it to the driver at every
-// synchronisation, and mapping a slot anew costs milliseconds).
+// synchronisation, and mapping a slot anew costs milliseconds).  The driver takes it for other slots of
+// the batch and for cudaMalloc before the device runs out, so live and kept memory stay within the
+// budget, but for what lies in chunks of 32 MB that a live solve shares.
 constexpr unsigned long long kKeepBytes = 4ull << 30;
 
 struct Slot {
