@@ -326,7 +326,8 @@ int upload_cellpar(setb_handle* h, const double* cell_par) {
 
 // Device memory of one flux call on host arrays: a stream and one block from a memory pool per device
 // that keeps at most 64 MB between calls (eight cudaMalloc / cudaFree pairs a call cost ~1 ms).  The
-// pool is stream-ordered, so calls from several threads do not see each other's blocks.
+// pool is stream-ordered, so calls from several threads do not see each other's blocks.  A device reset
+// leaves it as it is.
 cudaMemPool_t flux_pool(int device) {
     constexpr int kMaxDevices = 64;
     static std::mutex mu;

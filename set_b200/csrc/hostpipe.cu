@@ -15,49 +15,61 @@
 #include <new>
 #include <thread>
 
+#include <cudaTypedefs.h>
+
 #include "setb_internal.cuh"
 
 namespace sb {
 namespace {
 
+template <typename F> F driver_entry(const char* name, unsigned version) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPointByVersion(name, &p, version, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+        return reinterpret_cast<F>(p);
+    cudaGetLastError();
+    return nullptr;
+}
+
+// The calling thread's current context by an id that no other context of the process has had; 0: none, or
+// it cannot be told.
+unsigned long long context_id() {
+    static const auto current = driver_entry<PFN_cuCtxGetCurrent_v4000>("cuCtxGetCurrent", 4000);
+    static const auto id_of = driver_entry<PFN_cuCtxGetId_v12000>("cuCtxGetId", 12000);
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    return current && id_of && current(&c) == CUDA_SUCCESS && c && id_of(c, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 constexpr size_t kSlotBytes = 512 << 10;
 constexpr int kMaxThreads = 8;
-// Slots kept for later transfers: 8 MiB of pinned memory at most, given back when the last handle or
-// batch goes (host_pool_release; a program that makes flux calls alone keeps them).  Transfers that
-// overlap take more and give them back at once.
+// Slots kept for later transfers: 8 MiB of pinned memory a device at most, given back when its last handle
+// or batch goes (host_pool_release; a program that makes flux calls alone keeps them).  Transfers that
+// overlap take more and give them back at once.  A slot is used in the context it was allocated in alone: a
+// reset of the device releases it, and the context that follows has another id.
 constexpr int kKeepSlots = 2 * kMaxThreads;
+constexpr int kMaxDevices = 64;   // devices beyond that keep none
 
+struct Slot {
+    void* p;
+    unsigned long long ctx;
+};
 struct Pool {
     std::mutex mu;
-    void* free[kKeepSlots] = {};
+    Slot free[kKeepSlots] = {};
     int n = 0;
     long long owners = 0;
 };
-Pool g_pool;
+Pool g_pools[kMaxDevices];
 
-void* take_slot() {
-    {
-        std::lock_guard<std::mutex> lock(g_pool.mu);
-        if (g_pool.n > 0) return g_pool.free[--g_pool.n];
-    }
-    void* s = nullptr;
-    if (cudaHostAlloc(&s, kSlotBytes, cudaHostAllocPortable) != cudaSuccess) {
+Pool* pool_of_device() {
+    int d = 0;
+    if (cudaGetDevice(&d) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return s;
-}
-
-void give_slot(void* s) {
-    if (!s) return;
-    {
-        std::lock_guard<std::mutex> lock(g_pool.mu);
-        if (g_pool.n < kKeepSlots) {
-            g_pool.free[g_pool.n++] = s;
-            return;
-        }
-    }
-    cudaFreeHost(s);
+    return d >= 0 && d < kMaxDevices ? &g_pools[d] : nullptr;
 }
 
 bool pageable(const void* p) {
@@ -67,6 +79,40 @@ bool pageable(const void* p) {
         return true;
     }
     return a.type == cudaMemoryTypeUnregistered;
+}
+
+// `pool`, `ctx`: of the calling thread's device and context (null, 0: nothing is kept).
+void* take_slot(Pool* pool, unsigned long long ctx) {
+    if (pool && ctx) {
+        std::lock_guard<std::mutex> lock(pool->mu);
+        for (int k = pool->n - 1; k >= 0; k--)
+            if (pool->free[k].ctx == ctx) {
+                void* s = pool->free[k].p;
+                pool->free[k] = pool->free[--pool->n];
+                return s;
+            }
+    }
+    void* s = nullptr;
+    if (cudaHostAlloc(&s, kSlotBytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return s;
+}
+
+void give_slot(Pool* pool, unsigned long long ctx, void* s) {
+    if (!s) return;
+    if (pool && ctx) {
+        std::lock_guard<std::mutex> lock(pool->mu);
+        // a place, or that of a slot that went with its context
+        for (int k = 0; k < kKeepSlots; k++) {
+            if (k < pool->n && (pool->free[k].ctx == ctx || !pageable(pool->free[k].p))) continue;
+            pool->free[k] = Slot{s, ctx};
+            pool->n = std::max(pool->n, k + 1);
+            return;
+        }
+    }
+    cudaFreeHost(s);
 }
 
 // The copies of one call, handed out in slot-sized chunks.
@@ -183,17 +229,26 @@ cudaError_t copy_unstaged(const RowCopy& c, cudaStream_t s) {
 }  // namespace
 
 void host_pool_acquire() {
-    std::lock_guard<std::mutex> lock(g_pool.mu);
-    g_pool.owners++;
+    Pool* const pool = pool_of_device();
+    if (!pool) return;
+    std::lock_guard<std::mutex> lock(pool->mu);
+    pool->owners++;
 }
 
 void host_pool_release() {
+    Pool* const pool = pool_of_device();
+    if (!pool) return;
+    const unsigned long long ctx = context_id();
     void* drop[kKeepSlots];
     int n = 0;
     {
-        std::lock_guard<std::mutex> lock(g_pool.mu);
-        if (--g_pool.owners == 0)
-            for (; g_pool.n > 0; n++) drop[n] = g_pool.free[--g_pool.n];
+        std::lock_guard<std::mutex> lock(pool->mu);
+        if (--pool->owners == 0)
+            for (int k = pool->n - 1; k >= 0; k--)
+                if (pool->free[k].ctx == ctx) {
+                    drop[n++] = pool->free[k].p;
+                    pool->free[k] = pool->free[--pool->n];
+                }
     }
     for (int k = 0; k < n; k++) cudaFreeHost(drop[k]);
 }
@@ -228,9 +283,11 @@ cudaError_t copy_rows(const RowCopy* list, int count, cudaStream_t s) {
     const int want = (int)std::min<size_t>(std::min(kMaxThreads, hw), (total + (1u << 20) - 1) >> 20);
     void* slots[2 * kMaxThreads] = {};
     int pairs = 0;
+    Pool* const pool = pool_of_device();
+    const unsigned long long ctx = context_id();
     for (; pairs < want; pairs++) {
-        slots[2 * pairs] = take_slot();
-        slots[2 * pairs + 1] = take_slot();
+        slots[2 * pairs] = take_slot(pool, ctx);
+        slots[2 * pairs + 1] = take_slot(pool, ctx);
         if (!slots[2 * pairs] || !slots[2 * pairs + 1]) break;
     }
     if (pairs == 0) {
@@ -251,7 +308,7 @@ cudaError_t copy_rows(const RowCopy* list, int count, cudaStream_t s) {
         e = (cudaError_t)t.err.load();
         if (e != cudaSuccess) cudaStreamSynchronize(s);   // no copy may still use a slot
     }
-    for (void* p : slots) give_slot(p);
+    for (void* p : slots) give_slot(pool, ctx, p);
     return e;
 }
 

@@ -424,7 +424,7 @@ cudaError_t copy_rows_to_device(void* dev, const void* host, size_t hpitch, size
                                 const int32_t* perm, cudaStream_t s);
 cudaError_t copy_rows_to_host(void* host, size_t hpitch, const void* dev, size_t dpitch, size_t width, size_t n,
                               const int32_t* perm, cudaStream_t s);
-// Owners of the pinned slots kept between transfers (handles and batches).
+// Owners of the pinned slots kept between transfers on the calling thread's device (handles and batches).
 void host_pool_acquire();
 void host_pool_release();
 
