@@ -25,7 +25,7 @@
 #include <cmath>
 #include <cstring>
 #include <new>
-#include <numeric>
+#include <utility>
 #include <vector>
 
 #include "setb200.h"
@@ -681,7 +681,9 @@ int fl_create(FaceListDev** out, int64_t N, int64_t G, const double* cell_center
     if (rc) return rc;
     // Locality order: cells along the Morton curve of their centres, faces by their first cell, so
     // the cells a face gathers and the faces a cell gathers sit close in memory whatever the
-    // caller's numbering.  cperm[d] = caller's cell of device cell d; fperm likewise for faces.
+    // caller's numbering (ties by the caller's order).  cperm[d] = caller's cell of device cell d; fperm
+    // likewise for faces, which are counted into place: comparing them through the caller's random
+    // numbering was a third of the set-up.
     std::vector<int32_t> cperm((size_t)N), fperm((size_t)G), cnew((size_t)N), fnew((size_t)G);
     {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
@@ -690,7 +692,7 @@ int fl_create(FaceListDev** out, int64_t N, int64_t G, const double* cell_center
                 lo[a] = std::min(lo[a], cell_center_in[3 * c + a]);
                 hi[a] = std::max(hi[a], cell_center_in[3 * c + a]);
             }
-        std::vector<uint64_t> key((size_t)N);
+        std::vector<std::pair<uint64_t, int32_t>> key((size_t)N);
         for (int64_t c = 0; c < N; c++) {
             uint64_t code = 0;
             for (int a = 0; a < 3; a++) {
@@ -698,56 +700,28 @@ int fl_create(FaceListDev** out, int64_t N, int64_t G, const double* cell_center
                 const double u = (cell_center_in[3 * c + a] - lo[a]) / span;
                 code |= spread3((uint64_t)std::min(2097151.0, std::max(0.0, u * 2097151.0))) << a;
             }
-            key[c] = code;
+            key[c] = {code, (int32_t)c};
         }
-        std::iota(cperm.begin(), cperm.end(), 0);
-        std::stable_sort(cperm.begin(), cperm.end(), [&](int32_t x, int32_t y) { return key[x] < key[y]; });
-        for (int64_t d = 0; d < N; d++) cnew[cperm[d]] = (int32_t)d;
-        std::iota(fperm.begin(), fperm.end(), 0);
-        std::stable_sort(fperm.begin(), fperm.end(), [&](int32_t x, int32_t y) {
-            return cnew[gran_neighbour_in[2 * (int64_t)x] - 1] < cnew[gran_neighbour_in[2 * (int64_t)y] - 1];
-        });
-        for (int64_t d = 0; d < G; d++) fnew[fperm[d]] = (int32_t)d;
+        std::sort(key.begin(), key.end());
+        for (int64_t d = 0; d < N; d++) {
+            cperm[d] = key[d].second;
+            cnew[cperm[d]] = (int32_t)d;
+        }
+        std::vector<int32_t> at((size_t)N + 1, 0);   // first face of each cell, then its next free place
+        for (int64_t g = 0; g < G; g++) at[cnew[gran_neighbour_in[2 * g] - 1] + 1]++;
+        for (int64_t d = 0; d < N; d++) at[d + 1] += at[d];
+        for (int64_t g = 0; g < G; g++) {
+            fnew[g] = at[cnew[gran_neighbour_in[2 * g] - 1]]++;
+            fperm[fnew[g]] = (int32_t)g;
+        }
     }
+    // Cells, then faces, then the cells' face lists: what a face needs of its cells, and a cell of its
+    // faces, is read from the arrays already in locality order (a renumbered 96x80x64 box: this function
+    // on the host 390 ms; 760 with every array read through the caller's numbering and the sorts above by
+    // comparison, 690 with such sorts alone).
     auto cell_ref = [&](int32_t c1) { return cnew[c1 - 1]; };   // caller's 1-based -> device 0-based
     std::vector<double> cell_center((size_t)N * 3), inv_volume((size_t)N), geo((size_t)G * 4), normal4((size_t)G * 4);
     std::vector<int32_t> cell_gran((size_t)N * 6), type((size_t)G), nb((size_t)G * 4);
-    for (int64_t d = 0; d < G; d++) {
-        const int64_t g = fperm[d];
-        const int32_t s1 = gran_neighbour_in[2 * g], s2 = gran_neighbour_in[2 * g + 1], t = gran_type_in[g];
-        const int32_t ss1 = gran_neighbour_tvd_in[2 * g], ss2 = gran_neighbour_tvd_in[2 * g + 1];
-        const bool ghost = t == 4 || t == 5 || (t == 2 && s2 == -1);
-        // distances as the reference forms them each step (cuf_solvers.cuf:290-292, 362-372)
-        const double* gc = gran_center_in + 3 * g;
-        auto distance = [&](int32_t c) {
-            const double* x = cell_center_in + 3 * (int64_t)(c - 1);
-            const double r[3] = {gc[0] - x[0], gc[1] - x[1], gc[2] - x[2]};
-            return norm3(r);
-        };
-        const double df1 = distance(s1);
-        geo[4 * d] = df1;
-        const bool tvd = !ghost && ss1 >= 1 && ss2 >= 1;
-        if (tvd) {
-            const double df2 = distance(s2), dff1 = distance(ss1), dff2 = distance(ss2);
-            geo[4 * d + 1] = df1 / (df1 + df2);
-            geo[4 * d + 2] = df1 / (dff1 - df1);
-            geo[4 * d + 3] = df2 / (dff2 - df2);
-        }
-        const double* n = gran_normal_in + 3 * g;
-        for (int a = 0; a < 3; a++) normal4[4 * d + a] = n[a];
-        normal4[4 * d + 3] = gran_square_in[g];
-        nb[4 * d] = cell_ref(s1);
-        nb[4 * d + 1] = ghost ? nb[4 * d] : cell_ref(s2);
-        nb[4 * d + 2] = tvd ? cell_ref(ss1) : -1;
-        nb[4 * d + 3] = tvd ? cell_ref(ss2) : -1;
-        // the reference skips faces whose first cell lies inside its frozen core (:284)
-        const double* c1 = cell_center_in + 3 * (int64_t)(s1 - 1);
-        type[d] = (p->face_skip_radius > 0.0 && norm3(c1) < p->face_skip_radius) ? 0 : (t == 2 && !ghost ? kInner : t);
-        // physics 1: the reference's Lax flux on faces near the axis (cuf_solvers.cuf:293-295)
-        if (type[d] && p->physics == 1 && gc[0] > (double)0.22f && gc[1] < (double)0.1f &&
-            std::fabs(n[0]) < (double)0.1f)
-            type[d] |= kLaxFace;
-    }
     std::vector<unsigned char> flag((size_t)N);
     for (int64_t d = 0; d < N; d++) {
         const int64_t c = cperm[d];
@@ -757,13 +731,51 @@ int fl_create(FaceListDev** out, int64_t N, int64_t G, const double* cell_center
         flag[d] = ((p->cell_freeze_radius > 0.0 && norm3(x) < p->cell_freeze_radius) ? kFrozen : 0) |
                   ((p->r_src > 0.0 && r2 < p->r_src * p->r_src) ? kSource : 0);
         inv_volume[d] = 1.0 / cell_volume_in[c];
-        for (int f = 0; f < 6; f++) {   // the face, positive where this cell is its first neighbour
-            const int32_t j = cell_gran_in[6 * c + f];
-            if (j < 1) continue;
-            const int32_t jd = fnew[j - 1] + 1;
-            cell_gran[6 * d + f] = gran_neighbour_in[2 * (int64_t)(j - 1)] == (int32_t)(c + 1) ? jd : -jd;
-        }
     }
+    for (int64_t d = 0; d < G; d++) {
+        const int64_t g = fperm[d];
+        const int32_t s1 = gran_neighbour_in[2 * g], s2 = gran_neighbour_in[2 * g + 1], t = gran_type_in[g];
+        const int32_t ss1 = gran_neighbour_tvd_in[2 * g], ss2 = gran_neighbour_tvd_in[2 * g + 1];
+        const bool ghost = t == 4 || t == 5 || (t == 2 && s2 == -1);
+        const bool tvd = !ghost && ss1 >= 1 && ss2 >= 1;
+        int32_t* cells = nb.data() + 4 * d;
+        cells[0] = cell_ref(s1);
+        cells[1] = ghost ? cells[0] : cell_ref(s2);
+        cells[2] = tvd ? cell_ref(ss1) : -1;
+        cells[3] = tvd ? cell_ref(ss2) : -1;
+        // distances as the reference forms them each step (cuf_solvers.cuf:290-292, 362-372)
+        const double* gc = gran_center_in + 3 * g;
+        auto distance = [&](int32_t c) {
+            const double* x = cell_center.data() + 3 * (int64_t)c;
+            const double r[3] = {gc[0] - x[0], gc[1] - x[1], gc[2] - x[2]};
+            return norm3(r);
+        };
+        const double df1 = distance(cells[0]);
+        geo[4 * d] = df1;
+        if (tvd) {
+            const double df2 = distance(cells[1]), dff1 = distance(cells[2]), dff2 = distance(cells[3]);
+            geo[4 * d + 1] = df1 / (df1 + df2);
+            geo[4 * d + 2] = df1 / (dff1 - df1);
+            geo[4 * d + 3] = df2 / (dff2 - df2);
+        }
+        const double* n = gran_normal_in + 3 * g;
+        for (int a = 0; a < 3; a++) normal4[4 * d + a] = n[a];
+        normal4[4 * d + 3] = gran_square_in[g];
+        // the reference skips faces whose first cell lies inside its frozen core (:284)
+        const double* c1 = cell_center.data() + 3 * (int64_t)cells[0];
+        type[d] = (p->face_skip_radius > 0.0 && norm3(c1) < p->face_skip_radius) ? 0 : (t == 2 && !ghost ? kInner : t);
+        // physics 1: the reference's Lax flux on faces near the axis (cuf_solvers.cuf:293-295)
+        if (type[d] && p->physics == 1 && gc[0] > (double)0.22f && gc[1] < (double)0.1f &&
+            std::fabs(n[0]) < (double)0.1f)
+            type[d] |= kLaxFace;
+    }
+    for (int64_t d = 0; d < N; d++)
+        for (int f = 0; f < 6; f++) {   // the face, positive where this cell is its first neighbour
+            const int32_t j = cell_gran_in[6 * (int64_t)cperm[d] + f];
+            if (j < 1) continue;
+            const int32_t jd = fnew[j - 1];
+            cell_gran[6 * d + f] = nb[4 * (int64_t)jd] == (int32_t)d ? jd + 1 : -(jd + 1);
+        }
 
     FaceListDev* f = new (std::nothrow) FaceListDev();
     if (!f) return SETB_ENOMEM;
