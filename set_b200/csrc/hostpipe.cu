@@ -32,14 +32,23 @@ template <typename F> F driver_entry(const char* name, unsigned version) {
     return nullptr;
 }
 
-// The calling thread's current context by an id that no other context of the process has had; 0: none, or
-// it cannot be told.
-unsigned long long context_id() {
+// The calling thread's current context; null: none, or it cannot be told.
+CUcontext current_context() {
     static const auto current = driver_entry<PFN_cuCtxGetCurrent_v4000>("cuCtxGetCurrent", 4000);
-    static const auto id_of = driver_entry<PFN_cuCtxGetId_v12000>("cuCtxGetId", 12000);
     CUcontext c = nullptr;
+    return current && current(&c) == CUDA_SUCCESS ? c : nullptr;
+}
+// Makes the caller's context `c` (device `device`) current on a thread of the team.  The caller may have made
+// it by the driver API; cudaSetDevice would take the device's primary one, where its stream does not exist.
+cudaError_t enter_context(CUcontext c, int device) {
+    static const auto set = driver_entry<PFN_cuCtxSetCurrent_v4000>("cuCtxSetCurrent", 4000);
+    return c && set && set(c) == CUDA_SUCCESS ? cudaSuccess : cudaSetDevice(device);
+}
+// A context by an id that no other context of the process has had; 0: none, or it cannot be told.
+unsigned long long context_id(CUcontext c) {
+    static const auto id_of = driver_entry<PFN_cuCtxGetId_v12000>("cuCtxGetId", 12000);
     unsigned long long id = 0;
-    return current && id_of && current(&c) == CUDA_SUCCESS && c && id_of(c, &id) == CUDA_SUCCESS ? id : 0;
+    return c && id_of && id_of(c, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 constexpr size_t kSlotBytes = 512 << 10;
@@ -154,9 +163,10 @@ void move_rows(const RowCopy& t, char* slot, size_t r0, size_t m, bool in) {
     }
 }
 
-// One thread's share: two slots, so one is gathered or scattered while the other's copy runs.
-void work(Team* t, int device, void* s0, void* s1) {
-    cudaError_t e = cudaSetDevice(device);
+// One thread's share, in the caller's context: two slots, so one is gathered or scattered while the
+// other's copy runs.
+void work(Team* t, void* s0, void* s1) {
+    cudaError_t e = cudaSuccess;
     char* slot[2] = {static_cast<char*>(s0), static_cast<char*>(s1)};
     cudaEvent_t ev[2] = {nullptr, nullptr};
     for (int b = 0; b < 2 && e == cudaSuccess; b++) e = cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming);
@@ -199,6 +209,13 @@ void work(Team* t, int device, void* s0, void* s1) {
         if (ev[b]) cudaEventDestroy(ev[b]);
 }
 
+// The same on a thread of its own.
+void work_aside(Team* t, CUcontext ctx, int device, void* s0, void* s1) {
+    const cudaError_t e = enter_context(ctx, device);
+    if (e == cudaSuccess) work(t, s0, s1);
+    else t->err.store((int)e);
+}
+
 // A copy the driver makes by itself: known memory, or too little to be worth a slot.
 bool is_direct(const RowCopy& c) {
     return !c.perm && (c.n * c.width < (64u << 10) || c.dpitch > kSlotBytes || !pageable(c.host));
@@ -238,7 +255,7 @@ void host_pool_acquire() {
 void host_pool_release() {
     Pool* const pool = pool_of_device();
     if (!pool) return;
-    const unsigned long long ctx = context_id();
+    const unsigned long long ctx = context_id(current_context());
     void* drop[kKeepSlots];
     int n = 0;
     {
@@ -284,7 +301,8 @@ cudaError_t copy_rows(const RowCopy* list, int count, cudaStream_t s) {
     void* slots[2 * kMaxThreads] = {};
     int pairs = 0;
     Pool* const pool = pool_of_device();
-    const unsigned long long ctx = context_id();
+    CUcontext const current = current_context();
+    const unsigned long long ctx = context_id(current);
     for (; pairs < want; pairs++) {
         slots[2 * pairs] = take_slot(pool, ctx);
         slots[2 * pairs + 1] = take_slot(pool, ctx);
@@ -297,13 +315,13 @@ cudaError_t copy_rows(const RowCopy* list, int count, cudaStream_t s) {
         int started = 0;
         for (int k = 1; k < pairs; k++) {
             try {
-                th[started] = std::thread(work, &t, device, slots[2 * k], slots[2 * k + 1]);
+                th[started] = std::thread(work_aside, &t, current, device, slots[2 * k], slots[2 * k + 1]);
                 started++;
             } catch (const std::exception&) {   // no more threads: the others take its chunks
                 break;
             }
         }
-        work(&t, device, slots[0], slots[1]);
+        work(&t, slots[0], slots[1]);
         for (int k = 0; k < started; k++) th[k].join();
         e = (cudaError_t)t.err.load();
         if (e != cudaSuccess) cudaStreamSynchronize(s);   // no copy may still use a slot
