@@ -617,48 +617,47 @@ int32_t setb_batch_tune(setb_batch* b, int32_t reps, int32_t* lz_out, int32_t* g
             SB_TRY(cudaMemcpyAsync(&saved[s].second, b->slots[s].st, sizeof(DevStatus), cudaMemcpyDeviceToHost, b->stream));
         }
     SB_TRY(cudaStreamSynchronize(b->stream));
-    // one resident CTA per SM draws the tiles: more CTAs than that (a grid multiple) only queue
+    // one resident CTA per SM draws the tiles: more CTAs than that (a grid multiple) only queue, so the
+    // multiple is 1
     // 0: the members' own length (march_length), which goes on following them where none beats it
     const int lzs[] = {0, 8, 16, 32, 64, 1 << 20};
-    const int gms[] = {1};
     double best = 1e300;
     int best_lz = 0, best_gm = b->grid_mult;
     std::vector<int> timed;   // lengths that run
     cudaEvent_t e0, e1;
     SB_TRY(cudaEventCreate(&e0));
     SB_TRY(cudaEventCreate(&e1));
-    for (int lz : lzs)
-        for (int gm : gms) {
-            b->lz = lz ? lz : kDefaultLz;
-            b->lz_fixed = lz != 0;
-            b->grid_mult = gm;
-            b->dirty = true;
-            const int runs = march_length(b);
-            if (std::find(timed.begin(), timed.end(), runs) != timed.end()) continue;
-            timed.push_back(runs);
-            if (rebuild(b)) continue;
-            if (b->n_items == 0) continue;
-            auto launch_once = [&]() -> bool {
-                if (cudaMemsetAsync(b->d_queue, 0, 2 * sizeof(unsigned), b->stream) != cudaSuccess) return false;
-                return launch_items(b, 1, 3, b->d_queue) == SETB_OK && launch_items(b, 1, 2, b->d_queue + 1) == SETB_OK;
-            };
-            if (!launch_once()) continue;   // warm-up
-            cudaEventRecord(e0, b->stream);
-            bool ok = true;
-            for (int r = 0; r < reps && ok; r++) ok = launch_once();
-            cudaEventRecord(e1, b->stream);
-            cudaEventSynchronize(e1);
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            // longer marches only where they win clearly: the first stage alone is timed, and short tiles
-            // balance the second one better (6 grids of edges 48-112: first stage 0.49 ms with 8 and with
-            // 16 planes, a step 1.06 and 1.14 ms)
-            if (ok && ms / reps < 0.98 * best) {
-                best = ms / reps;
-                best_lz = lz;
-                best_gm = gm;
-            }
+    for (int lz : lzs) {
+        b->lz = lz ? lz : kDefaultLz;
+        b->lz_fixed = lz != 0;
+        b->grid_mult = 1;
+        b->dirty = true;
+        const int runs = march_length(b);
+        if (std::find(timed.begin(), timed.end(), runs) != timed.end()) continue;
+        timed.push_back(runs);
+        if (rebuild(b)) continue;
+        if (b->n_items == 0) continue;
+        auto launch_once = [&]() -> bool {
+            if (cudaMemsetAsync(b->d_queue, 0, 2 * sizeof(unsigned), b->stream) != cudaSuccess) return false;
+            return launch_items(b, 1, 3, b->d_queue) == SETB_OK && launch_items(b, 1, 2, b->d_queue + 1) == SETB_OK;
+        };
+        if (!launch_once()) continue;   // warm-up
+        cudaEventRecord(e0, b->stream);
+        bool ok = true;
+        for (int r = 0; r < reps && ok; r++) ok = launch_once();
+        cudaEventRecord(e1, b->stream);
+        cudaEventSynchronize(e1);
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, e0, e1);
+        // longer marches only where they win clearly: the first stage alone is timed, and short tiles
+        // balance the second one better (6 grids of edges 48-112: first stage 0.49 ms with 8 and with
+        // 16 planes, a step 1.06 and 1.14 ms)
+        if (ok && ms / reps < 0.98 * best) {
+            best = ms / reps;
+            best_lz = lz;
+            best_gm = 1;
         }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     b->lz = best_lz ? best_lz : kDefaultLz;

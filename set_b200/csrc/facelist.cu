@@ -591,16 +591,17 @@ __global__ void __launch_bounds__(kCellThreads) fl_cell_kernel(const FlView m, c
 
 template <int NSTATE, int ORDER, bool WANT_DT>
 void launch_face_o(const FlView& m, bool lax, double cfl, int n_disc, DevClock* clk, DevStatus* st, cudaStream_t s) {
-    constexpr bool HAS_FAST = NSTATE >= 2;
     const unsigned grid = (unsigned)((m.n_gran + kFaceThreads - 1) / kFaceThreads);
 #define SB_FACE(F, L) \
     launch_chained(fl_face_kernel<NSTATE, ORDER, WANT_DT, F, L>, grid, kFaceThreads, 0, s, m, cfl, n_disc, clk, st)
-    if (HAS_FAST && n_disc == 0) {
-        if (lax) SB_FACE(HAS_FAST, true);
-        else SB_FACE(HAS_FAST, false);
-    } else {
-        SB_FACE(false, true);
+    if constexpr (NSTATE >= 2) {
+        if (n_disc == 0) {
+            if (lax) SB_FACE(true, true);
+            else SB_FACE(true, false);
+            return;
+        }
     }
+    SB_FACE(false, true);
 #undef SB_FACE
 }
 
@@ -682,8 +683,8 @@ int fl_create(FaceListDev** out, int64_t N, int64_t G, const double* cell_center
     // Locality order: cells along the Morton curve of their centres, faces by their first cell, so
     // the cells a face gathers and the faces a cell gathers sit close in memory whatever the
     // caller's numbering (ties by the caller's order).  cperm[d] = caller's cell of device cell d; fperm
-    // likewise for faces, which are counted into place: comparing them through the caller's random
-    // numbering was a third of the set-up.
+    // likewise for faces, which are counted into place: sorts that compare through the caller's random
+    // numbering were half of the set-up.
     std::vector<int32_t> cperm((size_t)N), fperm((size_t)G), cnew((size_t)N), fnew((size_t)G);
     {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
