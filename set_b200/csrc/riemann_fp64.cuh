@@ -43,7 +43,8 @@ __device__ __forceinline__ double over_sqrt(double a, double x) {
 // clamped square roots do.  A side without pressure and field has a speed of exactly 0: the faces between
 // such sides at rest, which have no region, are told by it.  A NaN of either sign stays one, so the faces
 // of an invalid state are found.  Below the line the reciprocal square root gets 2^-328 (a finite seed; its
-// low word is that of 0, so the numerator costs one select more: 256^3 Heun 20.91 ms for six steps, 20.80 without).
+// low word is that of 0, so the numerator costs one select more: 256^3 Heun 20.91 ms for six steps,
+// 20.80 without).
 __device__ __forceinline__ double sqrt_ratio(double x, double y) {
     const bool none = x < 0x1p-328;
     return over_sqrt(none ? 0.0 : x, y * (none ? 0x1p-328 : x));

@@ -544,14 +544,19 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
     }
     __syncthreads();   // the first interval converts into the slot of plane k0-2
 
-    // Bits r: this thread's z, x and y face is a face of the grid.  Bits 4 + r: and no other tile counts it.
-    // Where the grid goes on, the z face below the chunk, the east x faces and the y faces above the last row
-    // are the neighbouring tiles', in dt candidates and diagnostics.  (256^3 Heun 20.97 ms for six steps; with
-    // the conditions formed at each face 21.1-21.2, without them 20.94.)
-    unsigned faces = own ? 0x11u : 0u;
-    if (rows ? gi <= g.nx && gj < g.ny : lane < TY && i0 + TX <= g.nx && j0 + lane < g.ny)
-        faces |= rows || i0 + TX == g.nx ? 0x22u : 0x02u;
-    if (gi < g.nx && gj <= g.ny) faces |= rows || gj == g.ny ? 0x44u : 0x04u;
+    // A face that another tile computes too (where the grid goes on: the z face below the chunk, the east x
+    // faces and the y faces above the last row) enters dt candidates and diagnostics in one of the two only.
+    // Plain and delta forms: bit r, this thread's z, x or y face is one that this tile counts (256^3 Heun
+    // 20.82 ms for six steps; with the conditions formed at each face 21.1-21.2, behind warp votes 21.46,
+    // with every face counted 20.95; delta 160x131x192 6.77 / 6.9 / 7.09 / 6.73).  The mixed form has no
+    // register for the bits: it asks behind a vote, where there is something to count (count_face; six-grid
+    // ensemble 227 ms, with the bits 232, with every face counted 228; 384^3 32.3 / 32.2 / 32.5).
+    unsigned faces = 0;
+    if constexpr (P != 1) {
+        faces = own ? 1u : 0u;
+        if (rows ? gi <= g.nx && gj < g.ny : lane < TY && i0 + TX == g.nx && j0 + lane < g.ny) faces |= 2u;
+        if (gi < g.nx && (rows ? gj <= g.ny : gj == g.ny)) faces |= 4u;
+    }
 
     // Flux sums of the plane in progress, natural component order.  FP64 fluxes: acc is the
     // area-weighted sum so far (starting with minus the z flux below); FP32 fluxes: the x
@@ -564,6 +569,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
         for (int r = 0; r < 3; r++) {   // z face k-1/2, x faces, y faces
             if (r == 0 ? !rows : k == k1) continue;
             int axis, fxx, fyy;
+            bool real;   // counted by this tile (mixed form: a face of the grid)
             double sq, idist;   // face area and 1/dist of the axis
             RT q1[8], q2[8];
             if (r == 0) {
@@ -594,6 +600,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
                         }
                     }
                 }
+                real = P == 1 ? own : (faces & 1u) && (k > k0 || k0 == kb);
             } else if (r == 1) {
                 axis = 0;
                 sq = g.square[0];
@@ -602,6 +609,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
                 fyy = rows ? warp : min(lane, TY - 1);
                 const RG* b = ring + ring_slot(k) * 8 * PLANE + (fyy + 2) * HX + fxx;
                 face_states<0, PLANE, P, ORDER>(b, b + 1, b + 2, b + 3, q1, q2);
+                real = P == 1 ? (rows || lane < TY) && i0 + fxx <= g.nx && j0 + fyy < g.ny : (faces & 2u) != 0;
             } else {
                 axis = 1;
                 sq = g.square[1];
@@ -610,9 +618,18 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
                 fyy = warp;
                 const RG* b = ring + ring_slot(k) * 8 * PLANE + cc - 2 * HX;
                 face_states<1, PLANE, P, ORDER>(b, b + HX, b + 2 * HX, b + 3 * HX, q1, q2);
+                real = P == 1 ? gi < g.nx && gj <= g.ny : (faces & 4u) != 0;
             }
-            const bool real = (faces >> (4 + r) & 1u) && (r != 0 || k > k0 || k0 == kb);
-            if (real && (sb_neg(q1[0]) || sb_neg(q2[0]))) n_recon++;
+            auto count_face = [&](int which) {   // mixed form
+                if (real && (r == 0 ? k > k0 || k0 == kb : rows || (r == 1 ? i0 + TX == g.nx : gj == g.ny)))
+                    atomicAdd(&cnt[which], 1ull);
+            };
+            const bool recon = sb_neg(q1[0]) || sb_neg(q2[0]);
+            if constexpr (P == 1) {
+                if (__any_sync(0xffffffffu, recon) && recon) count_face(2);
+            } else {
+                if (real && recon) n_recon++;
+            }
             int fl;
             double sl, sr;
             RT F[8];
@@ -650,7 +667,7 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
                 }
                 sl = (double)SL;
                 sr = (double)SR;
-                redone = P == 1 && (faces >> r & 1u) && (fl & kFlagStar);
+                redone = P == 1 && real && (fl & kFlagStar);
             }
             if (P == 1) {
 #pragma unroll
@@ -697,17 +714,20 @@ __device__ __forceinline__ void run_tile(const StageArgs& A, const CUtensorMap* 
                         sr = f.sr;
 #pragma unroll
                         for (int v = 0; v < 8; v++) F[v] = (RT)(f.F[face_perm_dyn(axis, v)] * sq);
-                        if (real) n_redo++;
+                        count_face(4);
                     }
                 }
             }
             // a face no wave-fan region matched gets a zero flux; the warp vote keeps the (never
             // taken in a valid state) zeroing out of the common path
-            if (__any_sync(0xffffffffu, fl & kFlagWave) && (fl & kFlagWave) && !(P == 1 && redone)) {
+            if (__any_sync(0xffffffffu, fl & kFlagWave) && (fl & kFlagWave)) {
+                if (!(P == 1 && redone)) {
 #pragma unroll
-                for (int v = 0; v < 8; v++) F[v] = RT(0);
+                    for (int v = 0; v < 8; v++) F[v] = RT(0);
+                }
+                if (P == 1) count_face(3);
             }
-            if ((fl & kFlagWave) && real) n_wave++;
+            if (P != 1 && (fl & kFlagWave) && real) n_wave++;
             // compare-and-select maxima (the library fmax of doubles is a far longer sequence); a NaN
             // speed is skipped, as fmax would skip it
             if (WANT_DT && real) rate = sb_max(rate, sb_max(fabs(sl), fabs(sr)) * idist);
