@@ -131,7 +131,8 @@ int shape_index(int precision, int shape) { return precision == 1 ? 1 + shape : 
 // one wave waits for them; with more waves the SMs that draw them take fewer tiles, where the last
 // wave has room.  With the drag counted, a stage of 64^3 took 62 us (mixed, 84 without) and 69 (delta,
 // 99), of 96^3 133 (173) and 170 (232), plain 96^3 120 (125); long marches that two CTAs share an
-// SM for hide it (mixed 256^3: 1.47 ms in one wave of 7-row tiles).
+// SM for hide it at first (mixed 256^3, one wave of 7-row tiles: stage 1 1.46 ms from the initial state,
+// 1.61 over 200 steps, in which the tiles that recompute grow).
 Tiling sb::choose_tiling(const GridGeom& g, int sm_count, int precision) {
     const double drag = precision == 0 ? 0.3 : (precision == 1 ? 0.9 : 0.7);
     const int nz = plane_end(g) - plane_begin(g);   // planes the stage kernels update

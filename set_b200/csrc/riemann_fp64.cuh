@@ -1,8 +1,8 @@
 // riemann_fp64.cuh -- the plain form's FP64 HLLD / HLLC flux and MUSCL face states, written for the
 // instruction budget of the stage kernel, which is bound by instruction issue and the latency of
-// dependent FP64 operations (FP64 pipe ~45 % busy, issue ~52 %, HBM ~15 %).  With it the kernel
-// issues 62 warp instructions per cell and stage instead of 81 (950 FP64 operations per cell instead
-// of 1050): 256^3 stage 1 / 2 2.04 / 2.15 -> 1.64 / 1.77 ms, and 2.31 / 2.44 ms with the former
+// dependent FP64 operations (FP64 pipe 44-46 % busy, issue 53-54 %, HBM 21-29 % at 256^3).  With it the kernel
+// issues 61-63 warp instructions per cell and stage instead of 84-86 (825-834 FP64 operations per cell
+// instead of 1006-1016): 256^3 stage 1 / 2 2.04 / 2.15 -> 1.64 / 1.77 ms, and 2.31 / 2.44 ms with the former
 // tile split; field-free HLLC 203x117x161 0.538 / 0.586 -> 0.390 / 0.430 ms.
 //
 // The same formulas and the same wave-fan selection as riemann<double, NSTATE, false, false, true,
