@@ -58,6 +58,23 @@ def test_faces_of_invalid_cells(shape, n_state, precision):
     assert redo[0] == redo[1] and (redo[0] > 0) == (precision > 0)
 
 
+@pytest.mark.parametrize("shape", [(64, 33, 8), (32, 11, 4), (96, 45, 7), (64, 28, 9)])
+@pytest.mark.parametrize("precision", [0, 1, 2])
+def test_faces_on_the_grid_s_end(shape, precision):
+    """Grids that end where tiles end (11, 15 and 7 rows): the end faces are the last tiles' own."""
+    nx, ny, nz = shape
+    inflow = S.lism_prim(u=(0.1, 0.3, 0.2))
+    cp = np.zeros((nx * ny * nz, 16))
+    cp[:, :8] = inflow
+    for i, j, k in ((nx - 1, ny - 1, nz - 1), (nx - 1, 5, 0), (3, ny - 1, nz // 2), (0, 0, nz - 1)):
+        cp[i + nx * (j + ny * k), 4] = np.nan
+    desc = S.cart_desc(shape, inflow=inflow, r_src=0.0, dt_init=1e-4)
+    want = oracle_count(desc, inflow, S.step_opts(scheme=1, order=1), cp)
+    with S.Solver(desc, cell_par=cp) as s:
+        s.step(1, S.step_opts(scheme=1, order=1, precision=precision), check=False)
+        assert s.status().n_wave_err == want == 24
+
+
 @pytest.mark.parametrize("shape", [(33, 23, 9), (70, 34, 5)])
 @pytest.mark.parametrize("n_state", [2, 3])
 def test_cold_faces_without_a_region(shape, n_state):
